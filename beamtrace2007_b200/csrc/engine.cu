@@ -37,6 +37,7 @@
 
 #include "bt_gpu.h"
 #include "engine_core.cuh"
+#include "group_core.cuh"
 #include "serve_engine.h"
 
 using namespace btg;
@@ -62,6 +63,7 @@ void setErr(const char* fmt, ...) {
   } while (0)
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr int kClipCtas = 6;
 constexpr int kWarps = 4;
 constexpr int kThreads = 32 * kWarps;
 constexpr double kFixVis = 1099511627776.0;         // 2^40: visible fraction, fixed point
@@ -98,9 +100,10 @@ struct __align__(128) Counters {
   int head;                     // fetch cursor of the trace queue being drained
   int pad1[13];
   int clipCount;                // records waiting for a clip (from the bottom of the clip queue)
-  int clipHead;                 // fetch cursor of the clip queue (clips, then deferred outputs)
+  int clipHead;                 // fetch cursor of the clip records
   int outQ;                     // finished pieces waiting for output (from the top of the clip queue)
-  int pad2[13];
+  int outHead;                  // fetch cursor of those
+  int pad2[12];
 };
 
 // Per-root query: plane, tolerances, mode (WfRoot, cuda/wavefront.cu:80-86).
@@ -801,6 +804,244 @@ __device__ __noinline__ bool clipRecord(const RoundParams& p, SubBeam* recp, Sta
   return false;
 }
 
+// ---- a clip by a group of lanes ------------------------------------------
+
+// A record's fields other than its corners, the same in every lane of the
+// group that works on it.
+struct GroupRec {
+  unsigned long long trail;
+  uint32_t node;
+  int root, hit, cursor, depth, n, neg;
+};
+
+__device__ __forceinline__ int4 recWords(const GroupRec& r, bool second) {
+  if (second) return make_int4(r.hit, r.cursor, (r.depth & 0xffff) | ((r.n & 0xff) << 16) | ((r.neg & 0xff) << 24), 0);
+  return make_int4(int(unsigned(r.trail)), int(unsigned(r.trail >> 32)), int(r.node), r.root);
+}
+
+__device__ __forceinline__ void loadRec(const SubBeam* at, GroupRec& r, float4& X, float4& Y) {
+  const float4* f = reinterpret_cast<const float4*>(at);
+  X = f[0];
+  Y = f[1];
+  const int4 a = reinterpret_cast<const int4*>(at)[2], b = reinterpret_cast<const int4*>(at)[3];
+  r.trail = (unsigned long long)(unsigned(a.x)) | ((unsigned long long)(unsigned(a.y)) << 32);
+  r.node = uint32_t(a.z);
+  r.root = a.w;
+  r.hit = b.x;
+  r.cursor = b.y;
+  r.depth = int(short(b.z & 0xffff));
+  r.n = int(int8_t((b.z >> 16) & 0xff));
+  r.neg = int(int8_t((b.z >> 24) & 0xff));
+}
+
+// Writes a record whose corner k lies in lane k of the group (8 lanes, 64 bytes at once).
+__device__ __forceinline__ void storeRec8(SubBeam* at, const GroupRec& r, float x, float y) {
+  const int sub = Grp<8>::sub();
+  if (sub < 4) {
+    reinterpret_cast<float*>(at)[sub] = x;
+    reinterpret_cast<float*>(at)[4 + sub] = y;
+  } else if (sub < 6) {
+    reinterpret_cast<int4*>(at)[sub - 2] = recWords(r, sub == 5);
+  }
+}
+
+// Reserves `n` slots of queue `q` for each group of the warp (n the same in a
+// group's lanes) with one atomic; returns the group's first slot, or -1 (and
+// flags an error) if they do not fit, which the reservation rule rules out.
+__device__ __forceinline__ int groupAppend(const RoundParams& p, int q, int n) {
+  using W = Grp<8>;
+  int before = 0, total = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const int ng = __shfl_sync(kFull, n, 8 * g);
+    if (8 * g < W::base()) before += ng;
+    total += ng;
+  }
+  if (total == 0) return -1;
+  int at = 0;
+  if (laneId() == 0) at = atomicAdd(&p.ctr->count[q], total);
+  at = __shfl_sync(kFull, at, 0);
+  if (at + total > p.capacity) {
+    if (laneId() == 0) atomicExch(&p.ctr->error, 1);
+    return -1;
+  }
+  return n > 0 ? at + before : -1;
+}
+
+enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
+
+// Clips the records of a warp's four groups (act: the group has one): the
+// triangle at a record's cursor needs it.  Pieces go to the next round's trace
+// queue in consecutive slots; with Keep the first piece stays with the group
+// (r and v become it: kClipKept).  kClipUnchanged: nothing measurable changed
+// and the record goes on at its next triangle (r.cursor moved).
+// v: corner k in lane k (lanes past n - 1 repeat the last).
+//
+// Pass 1 (groupClip) logs the pieces and measures what changes status
+// (splitPass1), pass 2 makes them beams (splitPass2, EmitSink).
+template <int App, bool Keep>
+__device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, bool act, GroupRec& r, LanePoly& v,
+                                          const Query& q, float lightArea, const HitPlane& h, Stats& st) {
+  using W = Grp<8>;
+  constexpr bool Nearest = App == kAppPrimary;
+  const int sub = W::sub();
+  const bool lead = sub == 0;
+  TriRec t;
+  t.v0 = t.v1 = t.v2 = t.n = mk(0, 0, 0);
+  t.vi[0] = t.vi[1] = t.vi[2] = 0;
+  t.tri = -1;
+  if (act) {
+    const uint2 leaf = p.s.node[r.node];
+    t = loadRef(p.s, leaf.x + uint32_t(r.cursor));
+  }
+  Line L;
+  int flags;
+  V3 r0, r1, r2;
+  laneLines<8, Nearest>(q, t, h, L, flags, r0, r1, r2);
+  const int nl = !Nearest || h.tri >= 0 ? 4 : 3;
+  float newArea;
+  int slots0, slots1, count, five;
+  LanePoly v0 = v;
+  if (!act) v0.n = 0;
+  const bool ok = groupClip(q.eps, v0, L, nl, act, S, newArea, slots0, slots1, count, five);
+  bool commit = act && ok && newArea >= q.minArea;
+  int res = act && ok && !commit ? int(kClipUnchanged) : int(kClipGone);
+  if (res == kClipUnchanged) r.cursor += 1;
+  if (lead && act && ok) st.fiveSplits += five;
+  if (lead && act && !ok) {
+    killRoot(p, r.root);
+    liveSub(p, r.root, 1);
+  }
+  const int slots = slots0 + (Nearest ? slots1 : 0);
+  int fits = 1;
+  if (lead && commit) {
+    const int old = atomicAdd(&p.live[r.root], slots - 1);
+    if (old + slots - 1 > p.budget || !coverLive(p, r.root, old + slots - 1)) {
+      killRoot(p, r.root);
+      liveSub(p, r.root, slots);
+      fits = 0;
+    } else if (old + slots - 1 == 0) {
+      rootDone(p, r.root);  // every piece occluded: the root is finished
+    }
+  }
+  fits = W::shfl(fits, 0);
+  commit = commit && fits;
+  if (!__any_sync(kFull, commit)) return res;
+  // `slots` pieces at most: one may stay with the group, the rest take reserved queue slots
+  const int want = commit ? max(0, Keep ? slots - 1 : slots) : 0;
+  const int at = groupAppend(p, p.cur ^ 1, want);
+  const int reserved = at >= 0 ? want : 0;
+  SubBeam* dst = p.tq[p.cur ^ 1] + max(at, 0);
+  if (lead && commit) st.splits++;
+  __syncwarp();
+  int filled = 0, k = 0, half = 0;
+  bool kept = false;
+  LanePoly kv = v;
+  int khit = -1;
+  GroupRec o = r;
+  o.cursor = r.cursor + 1;
+  if (!commit) count = 0;
+  while (__any_sync(kFull, k < count)) {
+    const bool on = k < count;
+    LanePoly b;
+    b.n = 0;
+    b.x = b.y = 0.f;
+    bool clean = true, hitNow = false;
+    if (on) {
+      const int n5 = S.n[k];
+      hitNow = S.level[k] == 1;
+      clean = S.clean[k] != 0;
+      int src = sub;
+      b.n = n5;
+      if (n5 == 5) {  // pentagon: quad (0,1,2,3), then triangle (0,3,4)
+        clean = false;
+        b.n = half ? 3 : 4;
+        if (half && sub > 0) src = sub + 2;
+        if (lead && half == 0) st.fiveSplits++;
+        k += half;
+        half ^= 1;
+      } else {
+        ++k;
+      }
+      if (src < 5) {
+        b.x = S.lx[k - (n5 == 5 ? 1 - half : 1)][src];
+        b.y = S.ly[k - (n5 == 5 ? 1 - half : 1)][src];
+      }
+    }
+    const LanePoly raw = b;
+    if (__any_sync(kFull, on && !clean)) groupClean(b, on && !clean, q.eps);
+    const float A = groupArea(b.x, b.y, b.n);
+    const bool drop = on && (b.n < 3 || A < q.minArea);
+    if (__any_sync(kFull, drop)) {
+      const float a0 = groupArea(raw.x, raw.y, raw.n);
+      if (drop && lead) st.dropped += double(a0 < 0 ? -a0 : a0);
+    }
+    const int c3 = b.n > 3 ? 3 : 2;
+    const float x3 = W::shfl(b.x, c3), y3 = W::shfl(b.y, c3);
+    if (sub >= 3) {
+      b.x = x3;
+      b.y = y3;
+    }
+    const bool good = on && !drop;
+    const bool queued = good && (Nearest || !hitNow);
+    if (queued) {
+      if (Keep && !kept) {
+        kept = true;
+        kv = b;
+        khit = hitNow ? t.tri : r.hit;
+      } else if (filled < reserved) {
+        o.n = b.n;
+        o.hit = hitNow ? t.tri : r.hit;
+        storeRec8(dst + filled, o, b.x, b.y);
+        ++filled;
+      }
+    }
+    if (!Nearest) {
+      const bool occ = good && hitNow;
+      if (lead && occ) {
+        st.hits++;
+        st.beams++;
+      }
+      if (App == kAppPoint && __any_sync(kFull, occ)) {
+        PieceOut po;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          po.qx[i] = W::shfl(b.x, i);
+          po.qy[i] = W::shfl(b.y, i);
+        }
+        if (lead && occ) {
+          po.P = q.P;
+          po.n = b.n;
+          po.root = r.root;
+          po.tri = t.tri;
+          po.exclude = q.exclude;
+          po.lightArea = lightArea;
+          outputPieceCold<App>(p, &po);
+        }
+      }
+    }
+  }
+  // slivers dropped were counted in `slots` but never queued (nor kept): empty
+  // records (n = -1) in their slots; with no piece at all (slots = 0) there was
+  // no kept slot to give back: the record itself was already taken off above
+  if (commit) {
+    const int unused = reserved - filled + (Keep && slots > 0 && !kept ? 1 : 0);
+    o.n = -1;
+    o.hit = -1;
+    o.cursor = 0;
+    for (; filled < reserved; ++filled) storeRec8(dst + filled, o, 0.f, 0.f);
+    if (lead && unused > 0) liveSub(p, r.root, unused);
+    if (Keep && kept) {
+      res = kClipKept;
+      v = kv;
+      r.cursor += 1;
+      r.hit = khit;
+      r.n = kv.n;
+    }
+  }
+  return res;
+}
+
 // ---- round kernels ------------------------------------------------------
 
 // Admission: each lane sets up one root (claimed per warp under the queue
@@ -1025,64 +1266,144 @@ __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const 
   flushStats(p, st);
 }
 
-// Clip: one lane per record of the clip queue; pieces go to the next
+// Finished pieces, deferred by the trace kernel to the top of the clip queue
+// (the output step is long and only a few lanes finish per step): one lane
+// per piece.
+template <int App>
+__device__ __forceinline__ void drainOutputs(const RoundParams& p, int nOut) {
+  const int lane = laneId();
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&p.ctr->outHead, 32);
+    base = __shfl_sync(kFull, base, 0);
+    if (base >= nOut) break;
+    if (base + lane >= nOut) continue;
+    const SubBeam o = p.cq[p.capacity - 1 - (base + lane)];
+    if (uint32_t(o.root) >= uint32_t(p.rootCap) || o.n < 3 || o.n > 4) {
+      atomicExch(&p.ctr->error, 2);
+      continue;
+    }
+    PieceOut po;
+    float lightArea;
+    Query q;
+    loadRoot<App>(&p.roots[o.root], q, lightArea);
+    po.P = q.P;
+    for (int k = 0; k < 4; ++k) {
+      po.qx[k] = o.qx[k];
+      po.qy[k] = o.qy[k];
+    }
+    po.n = o.n;
+    po.root = o.root;
+    po.tri = o.hit;
+    po.exclude = q.exclude;
+    po.lightArea = lightArea;
+    outputPieceCold<App>(p, &po);
+  }
+}
+
+// Clip records fill the clip queue from the bottom, deferred outputs from
+// the top; together they are at most the round's trace records.
+__device__ __forceinline__ bool clipQueueFits(const RoundParams& p, int nClip, int nOut) {
+  if (int64_t(nClip) + nOut <= p.capacity) return true;
+  if (threadIdx.x == 0 && blockIdx.x == 0) atomicExch(&p.ctr->error, 1);
+  return false;
+}
+
+// Clip: eight lanes per record of the clip queue; pieces go to the next
 // round's trace queue.  A record whose clip changes nothing measurable
 // continues at its next triangle in the next round.
-template <int App, bool F64 = false>
+//
+// Bound: the chain of operations of one clip and, on full queues, instruction
+// issue.  A polygon has at most six vertices, so eight lanes hold one with a
+// vertex each: classifying, splitting and cleaning it are a few ballots and
+// shuffles, where one lane per clip unrolled every polygon step six times
+// behind selects (128 registers with spills, 8 of 32 lanes active, instruction
+// fetch its top stall).  73 registers, 25 KB of shared memory a CTA.  Frames,
+// one lane -> eight lanes per clip (B200): plant 512^2 21.8 -> 18.7 ms, plant
+// 333x217 at light scale 4 49.3 -> 42.1, displaced sphere 512^2 at scale 2
+// 66.8 -> 60.2, meeting room ids at 1024^2 16.8 -> 14.9.
+template <int App>
+__global__ void __launch_bounds__(kThreads, kClipCtas) clipKernel(const __grid_constant__ RoundParams p) {
+  __shared__ ClipScratch scratch[kThreads / 8];
+  using W = Grp<8>;
+  const int lane = laneId();
+  const int nClip = p.ctr->clipCount, nOut = p.ctr->outQ;
+  if (!clipQueueFits(p, nClip, nOut)) return;
+  ClipScratch& S = scratch[threadIdx.x >> 3];
+  Stats st;
+  st.clear();
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&p.ctr->clipHead, 4);
+    base = __shfl_sync(kFull, base, 0);
+    if (base >= nClip) break;
+    const int i = base + (lane >> 3);
+    bool act = i < nClip;
+    GroupRec r;
+    float4 X, Y;
+    loadRec(p.cq + min(i, nClip - 1), r, X, Y);
+    if (p.state[r.root] == kRootKilled) {
+      if (act && W::sub() == 0) liveSub(p, r.root, 1);
+      act = false;
+    }
+    Query q;
+    float lightArea;
+    loadRoot<App>(&p.roots[r.root], q, lightArea);
+    HitPlane h;
+    h.tri = r.hit;
+    h.A[0] = h.A[1] = h.A[2] = h.C = 0.f;
+    h.n = mk(0, 0, 0);
+    if (App == kAppPrimary && r.hit >= 0) {
+      V3 v0;
+      triNV(p.s, r.hit, h.n, v0);
+      hitPlane(q, h.n, v0, h.A, h.C);
+    }
+    LanePoly v;
+    const int c = W::sub();
+    v.x = c == 0 ? X.x : (c == 1 ? X.y : (c == 2 ? X.z : X.w));
+    v.y = c == 0 ? Y.x : (c == 1 ? Y.y : (c == 2 ? Y.z : Y.w));
+    v.n = r.n;
+    const int res = clipGroups<App, false>(p, S, act, r, v, q, lightArea, h, st);
+    if (__any_sync(kFull, res == kClipUnchanged)) {
+      const int at = groupAppend(p, p.cur ^ 1, res == kClipUnchanged ? 1 : 0);
+      if (at >= 0) storeRec8(p.tq[p.cur ^ 1] + at, r, v.x, v.y);
+    }
+    __syncwarp();
+  }
+  flushStats(p, st);
+  drainOutputs<App>(p, nOut);
+}
+
+// The clip with FP64 re-decision of band corners (eps_fp64): one lane per
+// record.
 // (At least 4 CTAs per SM, i.e. at most 128 registers: with its polygons
 // in registers the clip step would take 255 and run 2 CTAs per SM; 4 keeps
 // enough warps for its latency and spills little -- measured 3 and 6 too.)
-__global__ void __launch_bounds__(kThreads, 4) clipKernel(const __grid_constant__ RoundParams p) {
+template <int App>
+__global__ void __launch_bounds__(kThreads, 4) clipFp64Kernel(const __grid_constant__ RoundParams p) {
   const int lane = laneId();
-  // clip records fill the clip queue from the bottom, deferred outputs from
-  // the top; together they are at most the round's trace records
   const int nClip = p.ctr->clipCount, nOut = p.ctr->outQ;
-  if (int64_t(nClip) + nOut > p.capacity) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) atomicExch(&p.ctr->error, 1);
-    return;
-  }
-  const int n = nClip + nOut;
+  if (!clipQueueFits(p, nClip, nOut)) return;
   Stats st;
   st.clear();
   for (;;) {
     int base = 0;
     if (lane == 0) base = atomicAdd(&p.ctr->clipHead, 32);
     base = __shfl_sync(kFull, base, 0);
-    if (base >= n) break;
-    const int i = base + lane;
-    if (i < nClip) {
-      SubBeam rec = p.cq[i];
+    if (base >= nClip) break;
+    if (base + lane < nClip) {
+      SubBeam rec = p.cq[base + lane];
       Stats cs;
       cs.clear();
-      if (clipRecord<App, F64>(p, &rec, &cs)) {
+      if (clipRecord<App, true>(p, &rec, &cs)) {
         const int at = queueAppend(p, p.cur ^ 1, 1);
         if (at >= 0) p.tq[p.cur ^ 1][at] = rec;
       }
       addStats(st, cs);
-    } else if (i < n) {
-      const SubBeam o = p.cq[p.capacity - 1 - (i - nClip)];
-      if (uint32_t(o.root) >= uint32_t(p.rootCap) || o.n < 3 || o.n > 4) {
-        atomicExch(&p.ctr->error, 2);
-      } else {
-        PieceOut po;
-        float lightArea;
-        Query q;
-        loadRoot<App>(&p.roots[o.root], q, lightArea);
-        po.P = q.P;
-        for (int k = 0; k < 4; ++k) {
-          po.qx[k] = o.qx[k];
-          po.qy[k] = o.qy[k];
-        }
-        po.n = o.n;
-        po.root = o.root;
-        po.tri = o.hit;
-        po.exclude = q.exclude;
-        po.lightArea = lightArea;
-        outputPieceCold<App>(p, &po);
-      }
     }
   }
   flushStats(p, st);
+  drainOutputs<App>(p, nOut);
 }
 
 // Between rounds: the drained queues are emptied, completion is decided
@@ -1095,6 +1416,7 @@ __global__ void roundEndKernel(Counters* c, int cur, int numRoots) {
   c->clipCount = 0;
   c->clipHead = 0;
   c->outQ = 0;
+  c->outHead = 0;
   c->warpsOut = 0;
   c->rounds++;
   c->done = (c->rootNext >= numRoots && c->inflight == 0 && c->count[nxt] == 0) ? 1 : 0;
@@ -1675,8 +1997,7 @@ struct RoundRunner {
          : mode == kVoteLog ? gridFor(c, traceKernel<App, false, kVoteLog>)
          : wide             ? gridFor(c, traceKernel<App, false, kVoteFloat, 4>)
                             : gridFor(c, traceKernel<App, false>);
-    gC = mode == kVoteFp64 ? gridFor(c, clipKernel<App, App == kAppSoft>, kLogSmem)
-                           : gridFor(c, clipKernel<App>, kLogSmem);
+    gC = mode == kVoteFp64 ? gridFor(c, clipFp64Kernel<kAppSoft>, kLogSmem) : gridFor(c, clipKernel<App>);
     gF = mode == kVoteFp64 ? gridFor(c, traceKernel<App, true, kVoteFp64F<App>>, kLogSmem)
          : mode == kVoteLog ? gridFor(c, traceKernel<App, true, kVoteLog>, kLogSmem)
                             : gridFor(c, traceKernel<App, true>, kLogSmem);
@@ -1829,9 +2150,9 @@ struct RoundRunner {
           traceKernel<App, false><<<gT, kThreads, 0, c->stream>>>(p);
         if (events) cudaEventRecord(c->kev[2 * k + 1], c->stream);
         if (mode == kVoteFp64)
-          clipKernel<App, App == kAppSoft><<<gC, kThreads, kLogSmem, c->stream>>>(p);
+          clipFp64Kernel<kAppSoft><<<gC, kThreads, kLogSmem, c->stream>>>(p);
         else
-          clipKernel<App><<<gC, kThreads, kLogSmem, c->stream>>>(p);
+          clipKernel<App><<<gC, kThreads, 0, c->stream>>>(p);
         launches += admit ? 4 : 3;
       }
       roundEndKernel<<<1, 1, 0, c->stream>>>(c->dCtr, p.cur, n);

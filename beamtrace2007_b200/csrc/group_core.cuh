@@ -1,0 +1,415 @@
+// One sub-beam worked on by a group of lanes (device code only).
+//
+// A beam is four corner rays, a triangle test is up to four lines against
+// those corners, a clip polygon has up to six vertices: a group of lanes
+// takes a corner, a line or a vertex each, so a record's step is a few short
+// operations deep where one lane would loop over them.  What bounds these
+// steps is the chain of dependent operations per record (a frame's records
+// depend on their parents, and a warp of independent records spends most of
+// its instructions on 3-4 of its 32 lanes), not bytes.
+//
+// Every value is computed by the same IEEE single-precision operations in
+// the same order as in beam_math.cuh / engine_core.cuh, so decisions, pieces
+// and counters are bitwise the same; sums over vertices run in vertex order.
+//
+// All lanes of a warp run these functions together (full-mask shuffles and
+// ballots, no divergence between groups); `act` says whether a group takes
+// part, and the values of a group that does not are never used.
+#pragma once
+
+#include "engine_core.cuh"
+
+namespace btg {
+
+// --------------------------------------------------------- lanes of a group
+
+template <int G>
+struct Grp {
+  static __device__ __forceinline__ int lane() { return threadIdx.x & 31; }
+  static __device__ __forceinline__ int sub() { return threadIdx.x & (G - 1); }
+  static __device__ __forceinline__ int base() { return threadIdx.x & 31 & ~(G - 1); }
+  // the group's lanes for which `pred` holds, bit 0 = its first lane
+  static __device__ __forceinline__ unsigned ballot(bool pred) {
+    return (__ballot_sync(0xffffffffu, pred) >> base()) & (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u);
+  }
+  template <class T>
+  static __device__ __forceinline__ T shfl(T v, int src) {
+    return __shfl_sync(0xffffffffu, v, src, G);
+  }
+};
+
+// A record's triangle: the line this lane looks after (0-2: the edges, 3: the
+// depth line against the current hit or the far plane) and what lane 0 found
+// about the triangle.
+enum { kTriPlain = 1, kTriFront = 2 };  // not edge-on; D > 0
+
+// The beam's current hit (primary visibility).
+struct HitPlane {
+  float A[3], C;
+  V3 n;
+  int tri;
+};
+
+// Edge lines and the depth line of triangle t, one per lane (BeamCtx::triSetup
+// and closerLine, as testOne evaluates them).  `flags`: kTriPlain | kTriFront,
+// the same in all lanes of the group.  An edge line's sign -- the orientation
+// of the triangle -- is applied to the normalised line: division and square
+// root are symmetric in it.  Lane 3 without a depth line (primary, no hit
+// yet) holds a line that every corner is inside of.
+template <int G, bool Nearest>
+__device__ __forceinline__ void laneLines(const Query& q, const TriRec& t, const HitPlane& h, Line& L, int& flags,
+                                          V3& r0, V3& r1, V3& r2) {
+  const int e = threadIdx.x & 3;
+  r0 = sub(t.v0, q.P.O);
+  r1 = sub(t.v1, q.P.O);
+  r2 = sub(t.v2, q.P.O);
+  const V3 ri = e == 0 ? r0 : (e == 1 ? r1 : r2), rj = e == 0 ? r1 : (e == 1 ? r2 : r0);
+  const bool fwd = e == 0 ? t.vi[0] < t.vi[1] : (e == 1 ? t.vi[1] < t.vi[2] : t.vi[2] < t.vi[0]);
+  V3 m = cross(fwd ? ri : rj, fwd ? rj : ri);
+  if (!fwd) m = neg(m);
+  int fl = 0;
+  {
+    const float D = dot(r2, m);  // lane 0's is the triangle's
+    if (notEdgeOn(D, m, r2)) fl |= kTriPlain;
+    if (D > 0) fl |= kTriFront;
+  }
+  flags = Grp<G>::shfl(fl, 0);
+  if (e == 3) m = t.n;
+  float a = dot(m, q.P.u), b = dot(m, q.P.v), c = dot(m, q.P.d);
+  float k = 0.f;  // a constant depth line's value
+  bool constant = false;
+  if (e == 3) {
+    const float TC = dot(t.n, r0);
+    constexpr bool far = !Nearest;
+    if (far || h.tri >= 0) {
+      const float CF = far ? q.farCq : h.C;
+      const V3 nF = far ? q.P.n : h.n;
+      const float A0 = far ? 0.f : h.A[0], A1 = far ? 0.f : h.A[1], A2 = far ? q.farCq : h.A[2];
+      const float cosang = dot(t.n, nF);
+      const float aC = TC < 0 ? -TC : TC, aF = CF < 0 ? -CF : CF;
+      const float scaleC = aC > aF ? aC : aF;
+      const float ca = cosang < 0 ? -cosang : cosang;
+      const float diff = TC - cosang * CF;
+      if (ca > 1 - kCoplanarCos && (diff < 0 ? -diff : diff) <= kCoplanarRel * scaleC) {
+        constant = true;
+        k = (!far && t.tri < h.tri) ? 1.f : -1.f;
+      }
+      const float sg = TC * CF > 0 ? 1.f : -1.f;
+      a = sg * (CF * a - TC * A0);
+      b = sg * (CF * b - TC * A1);
+      c = sg * (CF * c - TC * A2);
+    } else {
+      constant = true;
+      k = 1.f;
+    }
+  }
+  L = makeLine(a, b, c, q.ext);
+  if (e == 3) {
+    if (constant) L = Line{0.f, 0.f, k};
+  } else if (!(flags & kTriFront)) {
+    L.a = -L.a;
+    L.b = -L.b;
+    L.c = -L.c;
+  }
+}
+
+// -------------------------------------------------- polygons, a vertex a lane
+
+// Signed area (Poly::area): the terms are summed in vertex order.
+__device__ __forceinline__ float groupArea(float px, float py, int n) {
+  using W = Grp<8>;
+  const int nx = W::sub() + 1 == n ? 0 : W::sub() + 1;
+  const float xn = W::shfl(px, nx), yn = W::shfl(py, nx);
+  const float t = px * yn - xn * py;
+  float a = 0;
+#pragma unroll
+  for (int k = 0; k < kPolyMax; ++k) {
+    const float tk = W::shfl(t, k);
+    if (k < n) a += tk;
+  }
+  return a * 0.5f;
+}
+
+// A group's polygon in registers: this lane's vertex and the vertex count.
+struct LanePoly {
+  float x, y;
+  int n;
+};
+
+// cleanPoly, all vertices of a pass tested at once: vertices before the first
+// one to go are what the pass would have found them, so dropping that one and
+// going on at its place is the pass.
+struct CleanState {
+  bool run, changed;
+  int i0;
+};
+__device__ __forceinline__ void cleanBegin(CleanState& s, const LanePoly& p, bool act) {
+  s.run = act && p.n >= 3;
+  s.changed = false;
+  s.i0 = 0;
+}
+__device__ __forceinline__ void cleanStep(CleanState& s, LanePoly& p, float eps) {
+  using W = Grp<8>;
+  const int sub = W::sub();
+  const int h = sub == 0 ? p.n - 1 : sub - 1, j = sub + 1 >= p.n ? 0 : sub + 1;
+  const float xh = W::shfl(p.x, h), yh = W::shfl(p.y, h), xj = W::shfl(p.x, j), yj = W::shfl(p.y, j);
+  const float ex = xj - xh, ey = yj - yh, dx = p.x - xh, dy = p.y - yh;
+  const float len = sqrtf(ex * ex + ey * ey);
+  const float gapSq = dx * dx + dy * dy;
+  const float offLine = fabs_(ex * dy - ey * dx);
+  const bool goes = sub < p.n && (gapSq <= eps * eps || offLine <= eps * len);
+  const unsigned b = W::ballot(goes) & (0xffu << s.i0);
+  if (!__any_sync(0xffffffffu, s.run && b)) {  // no vertex goes in any group: a pass without a drop, or one more pass
+    s.run = s.run && s.changed;
+    s.changed = false;
+    s.i0 = 0;
+    return;
+  }
+  const float xs = W::shfl(p.x, sub + 1), ys = W::shfl(p.y, sub + 1);
+  if (s.run) {
+    if (b) {
+      const int k = __ffs(b) - 1;
+      if (sub >= k) {
+        p.x = xs;
+        p.y = ys;
+      }
+      --p.n;
+      s.changed = true;
+      s.i0 = k;
+      if (p.n < 3) s.run = false;
+    } else {
+      s.run = s.changed;
+      s.changed = false;
+      s.i0 = 0;
+    }
+  }
+}
+__device__ __forceinline__ void groupClean(LanePoly& p, bool act, float epsSplit) {
+  const float eps = epsSplit * 1e-3f;
+  CleanState s;
+  cleanBegin(s, p, act);
+  while (__any_sync(0xffffffffu, s.run)) cleanStep(s, p, eps);
+  if (act && p.n < 3) p.n = 0;
+}
+// two polygons of a group at once (the halves of a split)
+__device__ __forceinline__ void groupClean2(LanePoly& p, LanePoly& r, bool act, float epsSplit) {
+  const float eps = epsSplit * 1e-3f;
+  CleanState s, t;
+  cleanBegin(s, p, act);
+  cleanBegin(t, r, act);
+  while (__any_sync(0xffffffffu, s.run || t.run)) {
+    cleanStep(s, p, eps);
+    cleanStep(t, r, eps);
+  }
+  if (act && p.n < 3) p.n = 0;
+  if (act && r.n < 3) r.n = 0;
+}
+
+// Shared memory of one clipping group: the halves of a split on their way
+// from the lane that made a vertex to the lane that keeps it, the pending
+// pentagon halves (three corners each; at most one per line) and the pieces
+// of the first pass.
+//
+// Pieces: a polygon meets at most four lines (three edges and one depth
+// line); at each it gives one outside piece and at most two polygons that go
+// on (a pentagon in two), so f(l) = 1 + 2 f(l - 1) pieces, f(0) = 1: 31.
+constexpr int kGroupPieces = 31;
+struct __align__(16) ClipScratch {
+  float vx[2][8], vy[2][8];
+  float sx[5][3], sy[5][3];
+  int sline[5];
+  uint8_t level[kGroupPieces + 1], n[kGroupPieces + 1], clean[kGroupPieces + 1];
+  float lx[kGroupPieces][5], ly[kGroupPieces][5];
+};
+
+// Clips the group's beam by its lines, most-cutting edge first (clipTri), and
+// logs the pieces in push order.  L: the line of lanes 0-3 (nl of them used);
+// corners in lanes 0..n-1 of p.  Returns false if a piece or the pending list
+// overflowed.  newArea, slots0, slots1: AreaSink's sums; five: pentagons
+// split inside the clip.
+__device__ __forceinline__ bool groupClip(float eps, LanePoly p, const Line& L, int nl, bool act, ClipScratch& S,
+                                          float& newArea, int& slots0, int& slots1, int& count, int& five) {
+  using W = Grp<8>;
+  const int sub = W::sub();
+  const unsigned lt = (1u << sub) - 1u;
+  newArea = 0.f;
+  slots0 = slots1 = count = five = 0;
+  // the edges by how much of the beam lies inside, least first (stable)
+  int perm;
+  {
+    float score = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float dv = W::shfl(p.x, i) * L.a + W::shfl(p.y, i) * L.b + L.c;
+      const float pos = dv > 0.f ? dv : 0.f;
+      if (i == 0)
+        score = pos;
+      else if (i < 3)
+        score = score + pos;
+      else
+        score = score + (p.n == 4 ? pos : 0.f);
+    }
+    float s0 = W::shfl(score, 0), s1 = W::shfl(score, 1), s2 = W::shfl(score, 2);
+    int p0 = 0, p1 = 1, p2 = 2;
+    if (s1 < s0) {
+      const float t = s0;
+      s0 = s1;
+      s1 = t;
+      p0 = 1;
+      p1 = 0;
+    }
+    if (s2 < s1) {
+      p2 = p1;
+      p1 = 2;
+      s1 = s2;
+      if (s1 < s0) {
+        p1 = p0;
+        p0 = 2;
+      }
+    }
+    perm = p0 | (p1 << 4) | (p2 << 8) | (3 << 12);
+  }
+  bool ok = true, fail = false, clean = true;
+  bool run = act;
+  int li = 0, sp = 0;
+  while (__any_sync(0xffffffffu, run)) {
+    // the group's next line; past the last one the polygon is inside them all
+    const bool line = li < nl;
+    const int src = (perm >> (4 * (line ? li : 0))) & 15;
+    const float la = W::shfl(L.a, src), lb = W::shfl(L.b, src), lc = W::shfl(L.c, src);
+    const bool mine = sub < p.n;
+    const float d = la * p.x + lb * p.y + lc;
+    const int s = mine ? (d > eps ? 1 : (d < -eps ? -1 : 0)) : 0;
+    const unsigned bPos = W::ballot(s > 0), bNeg = W::ballot(s < 0);
+    const bool cut = run && line && bPos && bNeg;
+    const bool next = run && line && !bNeg;  // nothing outside this line
+    bool push = run && !cut && !next;
+    bool pop = push;
+    LanePoly o = p;           // what is pushed
+    int level = line ? 0 : 1;
+    bool oClean = clean;
+    if (__any_sync(0xffffffffu, cut)) {
+      // splitPoly: the vertices of both halves in emission order
+      const int nx = sub + 1 >= p.n ? 0 : sub + 1;
+      const int sn = W::shfl(s, nx);
+      const float dn = W::shfl(d, nx), xn = W::shfl(p.x, nx), yn = W::shfl(p.y, nx);
+      const bool cross = mine && s * sn < 0;
+      const unsigned bC = W::ballot(cross);
+      const unsigned all = p.n >= 8 ? 0xffu : (1u << p.n) - 1u;
+      const unsigned bIn = all & ~bNeg, bOut = all & ~bPos;
+      const int nIn = __popc(bIn) + __popc(bC), nOut = __popc(bOut) + __popc(bC);
+      const bool over = nIn > kPolyMax || nOut > kPolyMax;
+      if (cut && !over) {
+        const int at0 = __popc(bIn & lt) + __popc(bC & lt), at1 = __popc(bOut & lt) + __popc(bC & lt);
+        if (mine && s >= 0) {
+          S.vx[0][at0] = p.x;
+          S.vy[0][at0] = p.y;
+        }
+        if (mine && s <= 0) {
+          S.vx[1][at1] = p.x;
+          S.vy[1][at1] = p.y;
+        }
+        if (cross) {
+          // the crossing from the lexicographically smaller endpoint
+          const bool here = p.x < xn || (p.x == xn && p.y < yn);
+          const float da = here ? d : dn, db = here ? dn : d;
+          const float xa = here ? p.x : xn, xb = here ? xn : p.x;
+          const float ya = here ? p.y : yn, yb = here ? yn : p.y;
+          const float t = da / (da - db);
+          const float X = xa + t * (xb - xa);
+          const float Y = ya + t * (yb - ya);
+          const int k0 = at0 + (s >= 0 ? 1 : 0), k1 = at1 + (s <= 0 ? 1 : 0);
+          S.vx[0][k0] = X;
+          S.vy[0][k0] = Y;
+          S.vx[1][k1] = X;
+          S.vy[1][k1] = Y;
+        }
+      }
+      __syncwarp();
+      LanePoly in, out;
+      in.x = S.vx[0][sub];
+      in.y = S.vy[0][sub];
+      in.n = nIn;
+      out.x = S.vx[1][sub];
+      out.y = S.vy[1][sub];
+      out.n = nOut;
+      __syncwarp();
+      groupClean2(out, in, cut && !over, eps);
+      if (cut) {
+        if (over) {
+          fail = true;
+          run = false;
+        } else {
+          push = out.n >= 3;
+          o = out;
+          level = 0;
+          oClean = true;
+          if (in.n < 3) {
+            pop = true;
+          } else if (in.n == 5) {
+            // quad (0,1,2,3) goes on, triangle (0,3,4) waits
+            ++five;
+            if (sub == 0 || sub == 3 || sub == 4) {
+              const int k = sub == 0 ? 0 : sub - 2;
+              S.sx[sp][k] = in.x;
+              S.sy[sp][k] = in.y;
+            }
+            if (sub == 0) S.sline[sp] = li + 1;
+            ++sp;  // (at most one waits per line, so sp <= 4)
+            p = in;
+            p.n = 4;
+            clean = false;
+          } else {
+            p = in;
+            clean = true;
+          }
+        }
+      }
+    }
+    if (__any_sync(0xffffffffu, push)) {
+      const float area = groupArea(o.x, o.y, o.n);
+      if (push) {
+        if (o.n > 5) {
+          ok = false;
+        } else {
+          const int w = o.n == 5 ? 2 : 1;
+          if (level == 1) {
+            newArea += area;
+            slots1 += w;
+          } else {
+            slots0 += w;
+          }
+          if (sub < 5) {
+            S.lx[count][sub] = o.x;
+            S.ly[count][sub] = o.y;
+          }
+          if (sub == 0) {
+            S.level[count] = uint8_t(level);
+            S.n[count] = uint8_t(o.n);
+            S.clean[count] = oClean ? 1 : 0;
+          }
+          ++count;
+        }
+      }
+    }
+    ++li;
+    if (pop && run) {
+      if (sp == 0) {
+        run = false;
+      } else {
+        --sp;
+        li = S.sline[sp];
+        if (sub < 3) {
+          p.x = S.sx[sp][sub];
+          p.y = S.sy[sp][sub];
+        }
+        p.n = 3;
+        clean = false;
+      }
+    }
+    __syncwarp();
+  }
+  return ok && !fail;
+}
+
+}  // namespace btg

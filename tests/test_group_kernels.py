@@ -1,0 +1,73 @@
+"""The lane-group kernels (csrc/group_core.cuh) against the host emulator of
+the one-lane steps (tests/native/emu.cpp): the same pieces bit for bit and the
+same counters, over meshes whose clips give triangles, quads, pentagons and
+slivers, with rounds forced into full or tail kernels."""
+import numpy as np
+import pytest
+
+from conftest import piece_keys, scene
+
+pytestmark = pytest.mark.gpu
+
+COUNTERS = ["kd_steps", "leaf_visits", "tri_tests", "hits", "splits", "beams", "root_beams", "presplit_beams",
+            "five_splits", "climbs"]
+# never tail rounds; tail rounds whenever every root is admitted; records handed on early; the default
+MODES = [dict(tail_records=-1), dict(tail_records=1 << 30), dict(yield_pct=1), {}]
+
+
+def _soup(n=300, seed=5):
+    """Random interpenetrating triangles."""
+    from beamtrace2007_b200.renderer import PreparedScene
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    pos = (c + rng.normal(0, 0.35, (n, 3, 3))).reshape(-1, 3).astype(np.float32)
+    return PreparedScene(pos, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3))
+
+
+def _setup(name):
+    from beamtrace2007_b200.renderer import make_camera
+    if name == "soup":
+        ps = _soup()
+        return ps, make_camera((2.2, 1.1, 2.6), (0, 0, 0), 55.0, (0, 1, 0), 45, 37), (0.3, 3.0, 0.2), \
+            np.array([0.3, 3.0, 0.2, 0.9, 0, 0, 0, 0, 0.9])
+    s, ps = scene(name, **({"subdiv": 4} if name == "displaced_sphere" else {}))
+    v = s.views[0]
+    return ps, make_camera(v.eye, v.target, v.fov, s.up, 45, 37), s.point_light, s.light_array(1.5)
+
+
+def _counters(info, st):
+    return {k: (info[k], int(st[i])) for i, k in enumerate(COUNTERS) if info[k] != int(st[i])}
+
+
+@pytest.mark.parametrize("name", ["room", "plant", "displaced_sphere", "soup"])
+@pytest.mark.parametrize("mode", MODES, ids=["full", "tail", "yield", "default"])
+def test_pieces_and_counters_equal_emulator(name, mode, gpu):
+    from beamtrace2007_b200.renderer import GpuRenderer
+    from emu import Emulator
+    ps, cam, point, light = _setup(name)
+    em = Emulator(ps)
+    light_f = light.astype(np.float32)
+    with GpuRenderer(ps, budget=1 << 20, primary_budget=1 << 20, **mode) as g:
+        for tile in (3, 16):
+            prim = g.primary(cam, tile=tile)
+            info = g.last_info
+            pe, st = em.primary_tiles(cam, tile=tile)
+            assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
+            assert info["retried_roots"] == 0 and _counters(info, st) == {}
+            assert abs(info["dropped_area"] - float(st[10:11].view(np.float64)[0])) <= 1e-9
+        sh = g.point_shadows(cam, prim, point)
+        info = g.last_info
+        pe, st = em.point(cam, point, prim)
+        assert np.array_equal(piece_keys(sh), piece_keys(pe))
+        assert info["retried_roots"] == 0 and _counters(info, st) == {}
+        # shading points: the mean of each visible polygon's triangle corners, lifted to its plane
+        tri = prim.tri[:: max(1, len(prim) // 300)]
+        corners = ps.pos[ps.tris[tri].astype(np.int64)].astype(np.float64)
+        X = corners.mean(1).astype(np.float32)
+        N = ps.tri_normals[tri]
+        N = np.where((N.astype(np.float64) * (light[:3] - X)).sum(1, keepdims=True) < 0, -N, N).astype(np.float32)
+        r = g.soft_points(light, tri, X, N, exact=True, offset=ps.offset)
+        vis, G, st = em.soft_points(light_f, ps.offset, tri, X, N, exact=True)
+        assert r.info["retried_roots"] == 0 and _counters(r.info, st) == {}
+        # fixed point against double sums of the same pieces, each rounded to float
+        assert np.abs(r.vis - vis).max() <= 1e-6 and np.abs(r.E - G).max() <= 1e-6 * max(1.0, np.abs(G).max())
