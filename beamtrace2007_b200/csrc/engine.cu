@@ -64,6 +64,7 @@ void setErr(const char* fmt, ...) {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kClipCtas = 6;
+constexpr int kTailCtas = 4;  // (128 registers)
 constexpr int kWarps = 4;
 constexpr int kThreads = 32 * kWarps;
 constexpr double kFixVis = 1099511627776.0;         // 2^40: visible fraction, fixed point
@@ -806,14 +807,6 @@ __device__ __noinline__ bool clipRecord(const RoundParams& p, SubBeam* recp, Sta
 
 // ---- a clip by a group of lanes ------------------------------------------
 
-// A record's fields other than its corners, the same in every lane of the
-// group that works on it.
-struct GroupRec {
-  unsigned long long trail;
-  uint32_t node;
-  int root, hit, cursor, depth, n, neg;
-};
-
 __device__ __forceinline__ int4 recWords(const GroupRec& r, bool second) {
   if (second) return make_int4(r.hit, r.cursor, (r.depth & 0xffff) | ((r.n & 0xff) << 16) | ((r.neg & 0xff) << 24), 0);
   return make_int4(int(unsigned(r.trail)), int(unsigned(r.trail >> 32)), int(r.node), r.root);
@@ -1263,6 +1256,146 @@ __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const 
     }
   }
   if (!Fused && lane == 0) atomicAdd(&p.ctr->warpsOut, 1);
+  flushStats(p, st);
+}
+
+// Tail rounds: trace and clip in one kernel, eight lanes per record.  A group
+// walks its record, clips it where a triangle needs it and goes on with the
+// first piece (the others go to the next round), so a chain of splits
+// advances many levels per round.  A warp's four groups go through their steps
+// together, each time the step that most of them are at.
+//
+// Bound: the longest chain of walks and clips, one after the other.  With one
+// lane per record a step loops over four corners and three edges and a clip
+// over six vertices; here they lie side by side, which makes a step about a
+// third as long and a clip a tenth.  Tail rounds of a call, one lane -> eight
+// per record (B200): plant 512^2 3.0 -> 1.0 ms, meeting room ids 1024^2 7.2 ->
+// 4.5, 4801 points on the plant 3.4 -> 1.0, two retried roots of the displaced
+// sphere 54 -> 26.
+template <int App>
+__global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __grid_constant__ RoundParams p) {
+  __shared__ ClipScratch scratch[kThreads / 8];
+  constexpr int G = 8;
+  constexpr bool Nearest = App == kAppPrimary;
+  constexpr unsigned kLeads = 0x01010101u;
+  using W = Grp<G>;
+  const int lane = laneId(), sub = W::sub();
+  const bool lead = sub == 0;
+  const unsigned before = (1u << W::base()) - 1u;
+  const int nCur = min(p.ctr->count[p.cur], p.capacity);
+  const SubBeam* queue = p.tq[p.cur];
+  bool exhausted = nCur == 0;
+  // few records: spread over the warps, so that a warp's groups do not wait for each other's steps
+  const int warps = gridDim.x * kWarps;
+  const int most = max(1, min(32 / G, (nCur + warps - 1) / warps));
+  GroupWalk<G, Nearest> g;
+  g.idle();
+  float lightArea = 0.f;
+  int qRoot = -1;
+  Stats st;
+  st.clear();
+  for (;;) {
+    const unsigned mD = __ballot_sync(kFull, g.phase == kGDescend) & kLeads,
+                   mT = __ballot_sync(kFull, g.phase == kGTest) & kLeads,
+                   mC = __ballot_sync(kFull, g.phase == kGClimb) & kLeads,
+                   mS = __ballot_sync(kFull, g.phase == kGClip) & kLeads;
+    const int nD = __popc(mD), nT = __popc(mT), nC = __popc(mC), nS = __popc(mS), nBusy = nD + nT + nC + nS;
+    if (nBusy < most && (!exhausted || nBusy == 0)) {
+      const bool fin = g.phase == kGDone;
+      if (__any_sync(kFull, fin)) {
+        if (fin && lead) {
+          if (g.outTri >= 0) st.hits++;
+          st.beams++;
+          if (App == kAppSoft ? g.outTri < 0 : g.outTri >= 0) {  // soft keeps the visible light, the others the hits
+            PieceOut o;
+            o.P = g.q.P;
+            for (int i = 0; i < 4; ++i) {
+              o.qx[i] = g.cx[i];
+              o.qy[i] = g.cy[i];
+            }
+            o.n = g.r.n;
+            o.root = g.r.root;
+            o.tri = g.outTri;
+            o.exclude = g.q.exclude;
+            o.lightArea = lightArea;
+            outputPieceCold<App>(p, &o);
+          }
+          liveSub(p, g.r.root, 1);
+        }
+        if (fin) g.phase = kGIdle;
+        __syncwarp();
+      }
+      if (exhausted) break;
+      unsigned idle = __ballot_sync(kFull, g.phase == kGIdle) & kLeads;
+      for (int k = __popc(idle) - (most - nBusy); k > 0; --k) idle &= ~(1u << (31 - __clz(idle)));
+      const int ni = __popc(idle);
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&p.ctr->head, ni);
+      base = __shfl_sync(kFull, base, 0);
+      if (base + ni >= nCur) exhausted = true;
+      const int i = base + __popc(idle & before);
+      if (((idle >> W::base()) & 1u) && i < nCur) {
+        float4 X, Y;
+        loadRec(queue + i, g.r, X, Y);
+        if (uint32_t(g.r.root) >= uint32_t(p.rootCap) || g.r.node >= p.s.numNodes || g.r.n > 4) {
+          if (lead) atomicExch(&p.ctr->error, 2);  // a malformed record: report, never index with it
+        } else if (g.r.n < 0) {
+          // an empty slot of a clip's reservation
+        } else if (g.r.n == 0 || p.state[g.r.root] == kRootKilled) {
+          if (lead) liveSub(p, g.r.root, 1);  // a dropped sliver or an abandoned root
+        } else {
+          if (g.r.root != qRoot) {
+            loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);
+            qRoot = g.r.root;
+          }
+          g.cx[0] = X.x, g.cx[1] = X.y, g.cx[2] = X.z, g.cx[3] = X.w;
+          g.cy[0] = Y.x, g.cy[1] = Y.y, g.cy[2] = Y.z, g.cy[3] = Y.w;
+          g.begin(p.s, st);
+        }
+      }
+      __syncwarp();
+      continue;
+    }
+    if (nT >= nD && nT >= nC && nT >= nS) {
+      g.test(p.s, g.phase == kGTest, st);
+    } else if (nD >= nC && nD >= nS) {
+      g.descend(p.s, g.phase == kGDescend, st);
+    } else if (nC >= nS) {
+      g.climb(p.s, g.phase == kGClimb, st);
+    } else {
+      bool act = g.phase == kGClip;
+      if (act && p.state[g.r.root] == kRootKilled) {
+        if (lead) liveSub(p, g.r.root, 1);
+        g.phase = kGIdle;
+        act = false;
+      }
+      __syncwarp();
+      LanePoly v;
+      v.x = g.qx;
+      v.y = g.qy;
+      v.n = g.r.n;
+      const int res = clipGroups<App, true>(p, scratch[threadIdx.x >> 3], act, g.r, v, g.q, lightArea, g.h, st);
+      if (__any_sync(kFull, res == kClipKept)) {
+        float x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          x[i] = W::shfl(v.x, i);
+          y[i] = W::shfl(v.y, i);
+        }
+        if (res == kClipKept) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            g.cx[i] = x[i];
+            g.cy[i] = y[i];
+          }
+          g.begin(p.s, st);
+        }
+      }
+      if (act && res == kClipUnchanged) g.phase = g.r.cursor < int(g.nd.y >> 2) ? kGTest : kGClimb;
+      if (act && res == kClipGone) g.phase = kGIdle;
+    }
+  }
+  if (!lead) st.kdSteps = st.leafVisits = st.triTests = st.climbs = 0;  // (a group's lanes count the same steps)
   flushStats(p, st);
 }
 
@@ -2000,7 +2133,7 @@ struct RoundRunner {
     gC = mode == kVoteFp64 ? gridFor(c, clipFp64Kernel<kAppSoft>, kLogSmem) : gridFor(c, clipKernel<App>);
     gF = mode == kVoteFp64 ? gridFor(c, traceKernel<App, true, kVoteFp64F<App>>, kLogSmem)
          : mode == kVoteLog ? gridFor(c, traceKernel<App, true, kVoteLog>, kLogSmem)
-                            : gridFor(c, traceKernel<App, true>, kLogSmem);
+                            : gridFor(c, tailGroupKernel<App>);
     // tail rounds: every root admitted and fewer queued records than this
     // (default: a sixth of the trace grid's lanes, about two warps' worth per SM -- the fused kernel clips
     // inside the divergent walk, which only pays once the queue no longer fills the GPU)
@@ -2133,7 +2266,7 @@ struct RoundRunner {
         else if (mode == kVoteLog)
           traceKernel<App, true, kVoteLog><<<gF, kThreads, kLogSmem, c->stream>>>(p);
         else
-          traceKernel<App, true><<<gF, kThreads, kLogSmem, c->stream>>>(p);
+          tailGroupKernel<App><<<gF, kThreads, 0, c->stream>>>(p);
         if (events) cudaEventRecord(c->kev[2 * k + 1], c->stream);
         launches += 2;
         tailRounds++;

@@ -113,6 +113,292 @@ __device__ __forceinline__ void laneLines(const Query& q, const TriRec& t, const
   }
 }
 
+// ------------------------------------------------------ the walk of a record
+
+// A record's fields other than its corners, the same in every lane of the
+// group that works on it.
+struct GroupRec {
+  unsigned long long trail;
+  uint32_t node;
+  int root, hit, cursor, depth, n, neg;
+};
+
+// What a group does next.
+enum GroupPhase {
+  kGIdle = 0,     // no record
+  kGDescend = 1,  // at an inner node
+  kGTest = 2,     // a triangle of the leaf is pending
+  kGClimb = 3,    // the leaf (or a skipped cell) is done: pop the restart trail
+  kGDone = 4,     // the beam is finished: outTri
+  kGClip = 5      // the triangle at the cursor needs a clip
+};
+
+// A record being walked by a group of G lanes (4 or 8; lane k and lane k + 4
+// hold corner k & 3).  The steps are those of engine_core.cuh (descendStep,
+// climbStep, testOne) with the four corners, and the up to four lines of a
+// triangle, side by side; a step's corner comparisons are packed into one word
+// and the lanes' words combined by two shuffles.
+template <int G, bool Nearest>
+struct GroupWalk {
+  using W = Grp<G>;
+  GroupRec r;
+  Query q;
+  float cx[4], cy[4];  // every corner (the lines' votes)
+  float qx, qy;        // this lane's corner
+  float aw0, aw1, aw2; // |w| there
+  float farA, farC;
+  HitPlane h;
+  uint2 nd;            // record of r.node
+  Box box;             // its cell (while descending)
+  int phase, outTri;
+
+  static __device__ __forceinline__ unsigned all4(unsigned bits) {
+    bits &= __shfl_xor_sync(0xffffffffu, bits, 1);
+    return bits & __shfl_xor_sync(0xffffffffu, bits, 2);
+  }
+  // No record yet: values that the steps of other groups may compute with.
+  __device__ __forceinline__ void idle() {
+    r = GroupRec{0, 0, -1, -1, 0, 0, 0, 0};
+    q = Query{};
+    for (int k = 0; k < 4; ++k) cx[k] = cy[k] = 0.f;
+    qx = qy = aw0 = aw1 = aw2 = farA = farC = 0.f;
+    h = HitPlane{};
+    h.tri = -1;
+    nd = make_uint2(0, 3);
+    box = Box{};
+    phase = kGIdle;
+    outTri = -1;
+  }
+  __device__ __forceinline__ float aw(int a) const { return a == 0 ? aw0 : (a == 1 ? aw1 : aw2); }
+
+  __device__ __forceinline__ void setHit(int tri, V3 n, const float* A, float C) {
+    h.tri = tri;
+    h.n = n;
+    h.A[0] = A[0];
+    h.A[1] = A[1];
+    h.A[2] = A[2];
+    h.C = C;
+    farA = fabs_(qx * A[0] + qy * A[1] + A[2]);
+    farC = C < 0 ? -C : C;
+  }
+
+  // the cell of a node just entered: an inner one is descended, a leaf's
+  // triangles are next
+  __device__ __forceinline__ void enter(Stats& st) {
+    if (isLeaf(nd)) {
+      st.leafVisits++;
+      r.cursor = 0;
+      phase = (nd.y >> 2) > 0 ? kGTest : kGClimb;
+    } else {
+      phase = kGDescend;
+    }
+  }
+
+  // Takes up a record (expand, walkBegin); r, cx, cy and q are set.
+  __device__ __forceinline__ void begin(const SceneDev& s, Stats& st) {
+    const int c = threadIdx.x & 3;
+    qx = c == 0 ? cx[0] : (c == 1 ? cx[1] : (c == 2 ? cx[2] : cx[3]));
+    qy = c == 0 ? cy[0] : (c == 1 ? cy[1] : (c == 2 ? cy[2] : cy[3]));
+    const float w0 = qx * q.P.u.x + qy * q.P.v.x + q.P.d.x, w1 = qx * q.P.u.y + qy * q.P.v.y + q.P.d.y,
+                w2 = qx * q.P.u.z + qy * q.P.v.z + q.P.d.z;
+    const float s0 = w0 * ((r.neg & 1) ? -1.f : 1.f), s1 = w1 * ((r.neg & 2) ? -1.f : 1.f),
+                s2 = w2 * ((r.neg & 4) ? -1.f : 1.f);
+    aw0 = 0.f > s0 ? 0.f : s0;
+    aw1 = 0.f > s1 ? 0.f : s1;
+    aw2 = 0.f > s2 ? 0.f : s2;
+    nd = s.node[r.node];
+    h.tri = -1;
+    if (!Nearest) {
+      const float c0 = q.farCq < 0 ? -q.farCq : q.farCq;
+      farA = c0;
+      farC = c0;
+    } else {
+      farA = farC = 0.f;
+      if (r.hit >= 0) {
+        V3 nT, v0;
+        float A[3], C;
+        triNV(s, r.hit, nT, v0);
+        hitPlane(q, nT, v0, A, C);
+        setHit(r.hit, nT, A, C);
+      }
+    }
+    outTri = -1;
+    if (r.cursor < 0) {
+      box = loadBox(s, r.node);
+      enter(st);
+    } else {
+      phase = r.cursor < int(nd.y >> 2) ? kGTest : kGClimb;
+    }
+  }
+
+  // descendStep: into the child the beam enters first
+  __device__ __forceinline__ void descend(const SceneDev& s, bool act, Stats& st) {
+    const int a = int(nd.y & 3u);
+    const float sp = splitOf(nd);
+    const bool pos = !((r.neg >> a) & 1);
+    const float Ns = (pos ? 1.f : -1.f) * (sp - comp(q.P.O, a));
+    const uint32_t left = r.node + 1, right = nd.y >> 2;
+    uint2 ndLeft = nd, ndRight = nd;
+    if (act) {
+      ndLeft = s.node[left];
+      ndRight = s.node[right];
+    }
+    const float wa = aw(a);
+    unsigned bits = 0;
+#pragma unroll
+    for (int k = 1; k <= 2; ++k) {
+      const int c = a + k >= 3 ? a + k - 3 : a + k;
+      const bool p = !((r.neg >> c) & 1);
+      const float sc = p ? 1.f : -1.f, Oc = comp(q.P.O, c), lo = boxLo(box, c), hi = boxHi(box, c);
+      const float Nmin = sc * ((p ? lo : hi) - Oc), Nmax = sc * ((p ? hi : lo) - Oc);
+      const float lhs = aw(c) * Ns;
+      const float r0 = wa * Nmin, t0 = (fabs_(lhs) + fabs_(r0)) * kKdRel;
+      if (lhs < r0 - t0) bits |= 1u << (2 * k - 2);
+      const float r1 = wa * Nmax, t1 = (fabs_(lhs) + fabs_(r1)) * kKdRel;
+      if (lhs > r1 + t1) bits |= 1u << (2 * k - 1);
+    }
+    if (!Nearest || h.tri >= 0) {
+      const float lhs = farA * Ns, r0 = wa * farC, t0 = (fabs_(lhs) + fabs_(r0)) * kKdRel;
+      if (lhs > r0 + t0) bits |= 16u;
+    }
+    bits = all4(bits);
+    // decide: the first comparison that all corners pass (0 and 2: far child only)
+    const unsigned first = bits & (0u - bits);
+    const int dec = !(Ns > 0) ? int(kFar) : (bits == 0 ? int(kBoth) : ((first & 5u) ? int(kFar) : int(kNear)));
+    if (act) {
+      st.kdSteps++;
+      if (dec == kBoth) r.trail |= 1ull << r.depth;
+      r.depth++;
+      const bool goRight = dec == kFar ? pos : !pos;
+      r.node = goRight ? right : left;
+      nd = goRight ? ndRight : ndLeft;
+      if (goRight)
+        boxSetLo(box, a, sp);
+      else
+        boxSetHi(box, a, sp);
+      enter(st);
+    }
+  }
+
+  // climbStep: one pop of the restart trail
+  __device__ __forceinline__ void climb(const SceneDev& s, bool act, Stats& st) {
+    const bool go = act && r.trail != 0;
+    const int d = highestBit64(r.trail | 1ull);
+    uint32_t node = r.node, cs = r.node;
+    Box cb = box;
+    uint2 nc = nd;
+    if (go) {
+      for (int k = r.depth; k > d; --k) node = s.parent[node];
+      const uint2 nn = s.node[node];
+      cs = ((r.neg >> (nn.y & 3u)) & 1) ? node + 1 : (nn.y >> 2);
+      cb = loadBox(s, cs);
+      nc = s.node[cs];
+    }
+    float Nmin[3], Nmax[3];
+    bool miss = false;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const bool p = !((r.neg >> c) & 1);
+      const float sc = p ? 1.f : -1.f, Oc = comp(q.P.O, c);
+      Nmin[c] = sc * ((p ? cb.lo[c] : cb.hi[c]) - Oc);
+      Nmax[c] = sc * ((p ? cb.hi[c] : cb.lo[c]) - Oc);
+      if (Nmax[c] < 0) miss = true;
+    }
+    const float w[3] = {aw0, aw1, aw2};
+    unsigned bits = 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        if (c == e) continue;
+        const float lhs = w[e] * Nmax[c], r0 = w[c] * Nmin[e], t0 = (fabs_(lhs) + fabs_(r0)) * kKdRel;
+        if (lhs < r0 - t0) bits |= 1u << (3 * c + e);
+      }
+      if (!Nearest || h.tri >= 0) {
+        const float lhs = farA * Nmin[c], r0 = w[c] * farC, t0 = (fabs_(lhs) + fabs_(r0)) * kKdRel;
+        if (lhs > r0 + t0) bits |= 1u << (4 * c);  // (c == e above leaves these bits free)
+      }
+    }
+    bits = all4(bits);
+    if (go) {
+      st.climbs += uint32_t(r.depth - d);
+      r.trail &= (1ull << d) - 1;
+      if (miss || bits) {
+        r.node = node;
+        r.depth = d;
+      } else {
+        r.node = cs;
+        r.depth = d + 1;
+        r.cursor = -1;
+        box = cb;
+        nd = nc;
+        enter(st);
+      }
+    } else if (act) {
+      phase = kGDone;
+      outTri = Nearest ? h.tri : -1;
+    }
+  }
+
+  // testOne: the triangle at the cursor
+  __device__ __forceinline__ void test(const SceneDev& s, bool act, Stats& st) {
+    TriRec t;
+    t.v0 = t.v1 = t.v2 = t.n = mk(0, 0, 0);
+    t.vi[0] = t.vi[1] = t.vi[2] = 0;
+    t.tri = -1;
+    if (act) t = loadRef(s, nd.x + uint32_t(r.cursor));
+    Line L;
+    int flags;
+    V3 r0, r1, r2;
+    laneLines<G, Nearest>(q, t, h, L, flags, r0, r1, r2);
+    bool anyIn = false, anyOut = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float dv = cx[k] * L.a + cy[k] * L.b + L.c;
+      anyIn |= dv > q.eps;
+      anyOut |= dv < -q.eps;
+    }
+    const unsigned in = W::ballot(anyIn), out = W::ballot(anyOut);
+    const bool counted = act && t.tri != q.exclude && (flags & kTriPlain) && !(Nearest && q.cull && (flags & kTriFront));
+    const bool meets = counted && !(Nearest && h.tri == t.tri) && in == (1u << G) - 1u;
+    if (counted) st.triTests++;
+    const bool inside = meets && out == 0;
+    bool clip = meets && out != 0;
+    if (__any_sync(0xffffffffu, clip)) {
+      // separated: a side plane of the beam with all three vertices outside it
+      const int c = threadIdx.x & 3;
+      const float wx = qx * q.P.u.x + qy * q.P.v.x + q.P.d.x, wy = qx * q.P.u.y + qy * q.P.v.y + q.P.d.y,
+                  wz = qx * q.P.u.z + qy * q.P.v.z + q.P.d.z;
+      const int nx = (W::sub() & ~3) | ((c + 1) & 3);
+      const float vx = W::shfl(wx, nx), vy = W::shfl(wy, nx), vz = W::shfl(wz, nx);
+      const float sx = wy * vz - wz * vy, sy = wz * vx - wx * vz, sz = wx * vy - wy * vx;
+      const float sl = sqrtf(sx * sx + sy * sy + sz * sz);
+      bool o = r.n == 4 || c != 2;
+      const float e0 = sx * r0.x + sy * r0.y + sz * r0.z, e1 = sx * r1.x + sy * r1.y + sz * r1.z,
+                  e2 = sx * r2.x + sy * r2.y + sz * r2.z;
+      o = o && e0 < -(sl * (length(r0) * kEpsRel)) && e1 < -(sl * (length(r1) * kEpsRel)) &&
+          e2 < -(sl * (length(r2) * kEpsRel));
+      if (W::ballot(o)) clip = false;
+    }
+    if (act) {
+      if (clip) {
+        phase = kGClip;
+      } else if (!Nearest && inside) {
+        phase = kGDone;
+        outTri = t.tri;
+      } else {
+        if (inside) {
+          const float A[3] = {dot(t.n, q.P.u), dot(t.n, q.P.v), dot(t.n, q.P.d)};
+          setHit(t.tri, t.n, A, dot(t.n, r0));
+          r.hit = t.tri;
+        }
+        r.cursor += 1;
+        phase = r.cursor < int(nd.y >> 2) ? kGTest : kGClimb;
+      }
+    }
+  }
+};
+
 // -------------------------------------------------- polygons, a vertex a lane
 
 // Signed area (Poly::area): the terms are summed in vertex order.
