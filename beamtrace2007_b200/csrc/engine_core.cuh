@@ -355,15 +355,52 @@ BT_HD bool voteLine(const Query& q, const Beam& B, const Line& line, bool& allIn
   return anyIn;
 }
 
+BT_HD float max4abs(const float* v) {
+  return fmaxf(fmaxf(fabs_(v[0]), fabs_(v[1])), fmaxf(fabs_(v[2]), fabs_(v[3])));
+}
+
+// The votes on makeLine(a, b, c, ext): bit 0 some corner above eps, bit 1 some
+// corner below -eps.  Out of line (few tests need it, and the trace loop has to
+// fit the instruction caches), its arguments by value so that the caller's
+// corners stay in registers.
+BT_COLD int voteByLine(float x0, float x1, float x2, float x3, float y0, float y1, float y2, float y3, float a, float b,
+                       float c, float eps, float ext) {
+  const Line L = makeLine(a, b, c, ext);
+  const float d0 = x0 * L.a + y0 * L.b + L.c, d1 = x1 * L.a + y1 * L.b + L.c, d2 = x2 * L.a + y2 * L.b + L.c,
+              d3 = x3 * L.a + y3 * L.b + L.c;
+  return (d0 > eps || d1 > eps || d2 > eps || d3 > eps ? 1 : 0) |
+         (d0 < -eps || d1 < -eps || d2 < -eps || d3 < -eps ? 2 : 0);
+}
+
+// voteLine for makeLine(a, b, c, q.ext), which is made only when a corner is
+// too close to its band's edge to tell without.
+BT_HD bool voteCoefs(const Query& q, const Beam& B, float a, float b, float c, float maxX, float maxY, bool& allIn) {
+  bool in, out;
+  if (!voteUnscaled(B.qx, B.qy, a, b, c, maxX, maxY, q.eps, q.ext, in, out)) {
+    const int v = voteByLine(B.qx[0], B.qx[1], B.qx[2], B.qx[3], B.qy[0], B.qy[1], B.qy[2], B.qy[3], a, b, c, q.eps,
+                             q.ext);
+    in = v & 1;
+    out = (v & 2) != 0;
+  }
+  if (out) allIn = false;
+  return in;
+}
+BT_HD bool voteCloser(const Query& q, const Beam& B, const TriInfo& ti, const float* AF, float CF, V3 nF, int fId,
+                      bool& allIn) {
+  Line L;
+  if (!closerCoefs(ti, AF, CF, nF, fId, L)) return voteLine(q, B, L, allIn);
+  return voteCoefs(q, B, L.a, L.b, L.c, max4abs(B.qx), max4abs(B.qy), allIn);
+}
+
 // The tests after the three edges (depth line, far plane, inside, beam side)
 // of BeamCtx::classifyTri (beam_core.h:386-408); ti holds the full setup.
 BT_HD int classifyAfterEdges(const Query& q, const Beam& B, const TriInfo& ti, bool allIn) {
   if (q.mode == kModeNearest && B.hit >= 0) {
-    if (!voteLine(q, B, closerLine(q, ti, B.hitA, B.hitC, B.hitN, B.hit), allIn)) return kTriKeep;
+    if (!voteCloser(q, B, ti, B.hitA, B.hitC, B.hitN, B.hit, allIn)) return kTriKeep;
   }
   if (q.farIsPlane) {
     const float farA[3] = {0.f, 0.f, q.farCq};
-    if (!voteLine(q, B, closerLine(q, ti, farA, q.farCq, q.P.n, -1), allIn)) return kTriKeep;
+    if (!voteCloser(q, B, ti, farA, q.farCq, q.P.n, -1, allIn)) return kTriKeep;
   }
   if (allIn) return kTriAllIn;
   if (separated(q, B, ti)) return kTriKeep;
@@ -470,20 +507,42 @@ BT_HD int testOne(const SceneDev& s, const Query& q, SubBeam& r, Beam& B, Stats&
   if (B.hit == t.tri) return kStepContinue;
   const float sg = D > 0 ? 1.f : -1.f;
   bool allIn = true;
-  ti.edge[0] = makeLine(sg * dot(m0, q.P.u), sg * dot(m0, q.P.v), sg * dot(m0, q.P.d), q.ext);
-  if (EpsLog) logBand(q, B, ti.edge[0], t, 0, 1, sg, st);
-  if (F64 ? !voteLine64(q, B, ti.edge[0], t, 0, 1, sg, allIn, st) : !voteLine(q, B, ti.edge[0], allIn))
-    return kStepContinue;
-  const V3 m1 = edgePlane(ti.r, t.vi, 1, 2);
-  ti.edge[1] = makeLine(sg * dot(m1, q.P.u), sg * dot(m1, q.P.v), sg * dot(m1, q.P.d), q.ext);
-  if (EpsLog) logBand(q, B, ti.edge[1], t, 1, 2, sg, st);
-  if (F64 ? !voteLine64(q, B, ti.edge[1], t, 1, 2, sg, allIn, st) : !voteLine(q, B, ti.edge[1], allIn))
-    return kStepContinue;
-  const V3 m2 = edgePlane(ti.r, t.vi, 2, 0);
-  ti.edge[2] = makeLine(sg * dot(m2, q.P.u), sg * dot(m2, q.P.v), sg * dot(m2, q.P.d), q.ext);
-  if (EpsLog) logBand(q, B, ti.edge[2], t, 2, 0, sg, st);
-  if (F64 ? !voteLine64(q, B, ti.edge[2], t, 2, 0, sg, allIn, st) : !voteLine(q, B, ti.edge[2], allIn))
-    return kStepContinue;
+  if (Mode == kVoteFloat) {
+    // one body for the three edges (the trace loop has to fit the instruction
+    // caches): the corners of the triangle turn round under it
+    const float maxX = max4abs(B.qx), maxY = max4abs(B.qy);
+    V3 m = m0;
+    uint32_t i0 = t.vi[0], i1 = t.vi[1], i2 = t.vi[2];
+    BT_ROLL for (int e = 0;;) {
+      if (!voteCoefs(q, B, sg * dot(m, q.P.u), sg * dot(m, q.P.v), sg * dot(m, q.P.d), maxX, maxY, allIn))
+        return kStepContinue;
+      const V3 r0 = ti.r[0];
+      const uint32_t k0 = i0;
+      ti.r[0] = ti.r[1];
+      ti.r[1] = ti.r[2];
+      ti.r[2] = r0;
+      i0 = i1;
+      i1 = i2;
+      i2 = k0;
+      if (++e == 3) break;  // (round to the first corner again)
+      m = i0 < i1 ? cross(ti.r[0], ti.r[1]) : neg(cross(ti.r[1], ti.r[0]));
+    }
+  } else {
+    ti.edge[0] = makeLine(sg * dot(m0, q.P.u), sg * dot(m0, q.P.v), sg * dot(m0, q.P.d), q.ext);
+    if (EpsLog) logBand(q, B, ti.edge[0], t, 0, 1, sg, st);
+    if (F64 ? !voteLine64(q, B, ti.edge[0], t, 0, 1, sg, allIn, st) : !voteLine(q, B, ti.edge[0], allIn))
+      return kStepContinue;
+    const V3 m1 = edgePlane(ti.r, t.vi, 1, 2);
+    ti.edge[1] = makeLine(sg * dot(m1, q.P.u), sg * dot(m1, q.P.v), sg * dot(m1, q.P.d), q.ext);
+    if (EpsLog) logBand(q, B, ti.edge[1], t, 1, 2, sg, st);
+    if (F64 ? !voteLine64(q, B, ti.edge[1], t, 1, 2, sg, allIn, st) : !voteLine(q, B, ti.edge[1], allIn))
+      return kStepContinue;
+    const V3 m2 = edgePlane(ti.r, t.vi, 2, 0);
+    ti.edge[2] = makeLine(sg * dot(m2, q.P.u), sg * dot(m2, q.P.v), sg * dot(m2, q.P.d), q.ext);
+    if (EpsLog) logBand(q, B, ti.edge[2], t, 2, 0, sg, st);
+    if (F64 ? !voteLine64(q, B, ti.edge[2], t, 2, 0, sg, allIn, st) : !voteLine(q, B, ti.edge[2], allIn))
+      return kStepContinue;
+  }
   ti.n = t.n;
   ti.A[0] = dot(t.n, q.P.u);
   ti.A[1] = dot(t.n, q.P.v);

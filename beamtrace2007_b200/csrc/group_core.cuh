@@ -50,14 +50,14 @@ struct HitPlane {
   int tri;
 };
 
-// Edge lines and the depth line of triangle t, one per lane (BeamCtx::triSetup
-// and closerLine, as testOne evaluates them).  `flags`: kTriPlain | kTriFront,
-// the same in all lanes of the group.  An edge line's sign -- the orientation
-// of the triangle -- is applied to the normalised line: division and square
-// root are symmetric in it.  Lane 3 without a depth line (primary, no hit
-// yet) holds a line that every corner is inside of.
+// Edge lines and the depth line of triangle t, one per lane, before they are
+// normalised (BeamCtx::triSetup and closerLine, as testOne evaluates them):
+// true with the coefficients in L, or false with a constant line in L (lane 3:
+// a tie of coplanar surfaces, or no depth line -- primary, no hit yet --, which
+// every corner is inside of).  `flags`: kTriPlain | kTriFront, the same in all
+// lanes of the group.
 template <int G, bool Nearest>
-__device__ __forceinline__ void laneLines(const Query& q, const TriRec& t, const HitPlane& h, Line& L, int& flags,
+__device__ __forceinline__ bool laneCoefs(const Query& q, const TriRec& t, const HitPlane& h, Line& L, int& flags,
                                           V3& r0, V3& r1, V3& r2) {
   const int e = threadIdx.x & 3;
   r0 = sub(t.v0, q.P.O);
@@ -75,42 +75,30 @@ __device__ __forceinline__ void laneLines(const Query& q, const TriRec& t, const
   }
   flags = Grp<G>::shfl(fl, 0);
   if (e == 3) m = t.n;
-  float a = dot(m, q.P.u), b = dot(m, q.P.v), c = dot(m, q.P.d);
-  float k = 0.f;  // a constant depth line's value
-  bool constant = false;
+  L.a = dot(m, q.P.u);
+  L.b = dot(m, q.P.v);
+  L.c = dot(m, q.P.d);
   if (e == 3) {
-    const float TC = dot(t.n, r0);
     constexpr bool far = !Nearest;
-    if (far || h.tri >= 0) {
-      const float CF = far ? q.farCq : h.C;
-      const V3 nF = far ? q.P.n : h.n;
-      const float A0 = far ? 0.f : h.A[0], A1 = far ? 0.f : h.A[1], A2 = far ? q.farCq : h.A[2];
-      const float cosang = dot(t.n, nF);
-      const float aC = TC < 0 ? -TC : TC, aF = CF < 0 ? -CF : CF;
-      const float scaleC = aC > aF ? aC : aF;
-      const float ca = cosang < 0 ? -cosang : cosang;
-      const float diff = TC - cosang * CF;
-      if (ca > 1 - kCoplanarCos && (diff < 0 ? -diff : diff) <= kCoplanarRel * scaleC) {
-        constant = true;
-        k = (!far && t.tri < h.tri) ? 1.f : -1.f;
-      }
-      const float sg = TC * CF > 0 ? 1.f : -1.f;
-      a = sg * (CF * a - TC * A0);
-      b = sg * (CF * b - TC * A1);
-      c = sg * (CF * c - TC * A2);
-    } else {
-      constant = true;
-      k = 1.f;
+    if (!far && h.tri < 0) {
+      L = Line{0.f, 0.f, 1.f};
+      return false;
     }
+    TriInfo ti;
+    ti.tri = t.tri;
+    ti.n = t.n;
+    ti.A[0] = L.a;
+    ti.A[1] = L.b;
+    ti.A[2] = L.c;
+    ti.C = dot(t.n, r0);
+    const float AF[3] = {far ? 0.f : h.A[0], far ? 0.f : h.A[1], far ? q.farCq : h.A[2]};
+    return closerCoefs(ti, AF, far ? q.farCq : h.C, far ? q.P.n : h.n, far ? -1 : h.tri, L);
   }
-  L = makeLine(a, b, c, q.ext);
-  if (e == 3) {
-    if (constant) L = Line{0.f, 0.f, k};
-  } else if (!(flags & kTriFront)) {
-    L.a = -L.a;
-    L.b = -L.b;
-    L.c = -L.c;
-  }
+  const float sg = (flags & kTriFront) ? 1.f : -1.f;
+  L.a *= sg;
+  L.b *= sg;
+  L.c *= sg;
+  return true;
 }
 
 // ------------------------------------------------------ the walk of a record
@@ -350,13 +338,19 @@ struct GroupWalk {
     Line L;
     int flags;
     V3 r0, r1, r2;
-    laneLines<G, Nearest>(q, t, h, L, flags, r0, r1, r2);
-    bool anyIn = false, anyOut = false;
+    const bool line = laneCoefs<G, Nearest>(q, t, h, L, flags, r0, r1, r2);
+    bool anyIn = L.c > q.eps, anyOut = L.c < -q.eps;  // (a constant line's vote)
+    const bool known = !line || voteUnscaled(cx, cy, L.a, L.b, L.c, max4abs(cx), max4abs(cy), q.eps, q.ext, anyIn, anyOut);
+    if (__any_sync(0xffffffffu, act && !known)) {
+      // a corner too close to its band's edge: the line itself
+      const Line N = line ? makeLine(L.a, L.b, L.c, q.ext) : L;
+      anyIn = anyOut = false;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float dv = cx[k] * L.a + cy[k] * L.b + L.c;
-      anyIn |= dv > q.eps;
-      anyOut |= dv < -q.eps;
+      for (int k = 0; k < 4; ++k) {
+        const float dv = cx[k] * N.a + cy[k] * N.b + N.c;
+        anyIn |= dv > q.eps;
+        anyOut |= dv < -q.eps;
+      }
     }
     const unsigned in = W::ballot(anyIn), out = W::ballot(anyOut);
     const bool counted = act && t.tri != q.exclude && (flags & kTriPlain) && !(Nearest && q.cull && (flags & kTriFront));

@@ -533,3 +533,21 @@ EMU_API int emu_decide(const float* O, const float* p0, const float* u, const fl
   if (!(Ns > 0)) return -2;
   return decide(q, b, axis, Ns, box);
 }
+
+// The votes of four corners on the line makeLine(a, b, c, ext): out[0], out[1]
+// some corner above eps / below -eps by the line itself, and, if voteUnscaled
+// can tell (the result), out[2], out[3] what it says.  For the vote fuzz test.
+EMU_API int emu_vote(const float* qx, const float* qy, float a, float b, float c, float eps, float ext, int* out) {
+  const Line L = makeLine(a, b, c, ext);
+  out[0] = out[1] = 0;
+  for (int k = 0; k < 4; ++k) {
+    const float dv = qx[k] * L.a + qy[k] * L.b + L.c;
+    out[0] |= dv > eps;
+    out[1] |= dv < -eps;
+  }
+  bool in = false, below = false;
+  const int known = voteUnscaled(qx, qy, a, b, c, max4abs(qx), max4abs(qy), eps, ext, in, below);
+  out[2] = in;
+  out[3] = below;
+  return known;
+}
