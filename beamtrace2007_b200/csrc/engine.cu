@@ -179,6 +179,7 @@ struct RoundParams {
   int numRoots;
   int rootCap;  // size of the per-root arrays
   int yieldAt;  // exited trace warps at which the rest hand their records on (INT_MAX: never)
+  int tailMax;  // a tail round leaves a longer queue to the full rounds
   const int32_t* rootList;
   RootRec* roots;  // per-root query records
   int32_t* live;
@@ -1283,6 +1284,7 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
   const bool lead = sub == 0;
   const unsigned before = (1u << W::base()) - 1u;
   const int nCur = min(p.ctr->count[p.cur], p.capacity);
+  if (nCur > p.tailMax) return;  // (roundEndKernel keeps the queue)
   const SubBeam* queue = p.tq[p.cur];
   bool exhausted = nCur == 0;
   // few records: spread over the warps, so that a warp's groups do not wait for each other's steps
@@ -1541,7 +1543,14 @@ __global__ void __launch_bounds__(kThreads, 4) clipFp64Kernel(const __grid_const
 
 // Between rounds: the drained queues are emptied, completion is decided
 // (scheduleKernel's bookkeeping, cuda/wavefront.cu:327-345).
-__global__ void roundEndKernel(Counters* c, int cur, int numRoots) {
+// keepAbove: a tail round did not touch a queue longer than this; it stays as
+// it is, the tail rounds that follow in the batch find nothing to do, and the
+// host, which sees the counts after the batch, goes on with full rounds.
+__global__ void roundEndKernel(Counters* c, int cur, int numRoots, int keepAbove) {
+  if (c->count[cur] > keepAbove) {
+    c->rounds++;
+    return;
+  }
   const int nxt = cur ^ 1;
   if (c->count[nxt] > c->maxQueue) c->maxQueue = c->count[nxt];
   c->count[cur] = 0;
@@ -2062,6 +2071,11 @@ constexpr int64_t kWideSceneBytes = int64_t(16) << 20;
 // holds at most half a record per root (long walks, few splits: point
 // shadows of a sparse scene) goes to tail rounds at once.
 constexpr int kFirstRounds = 2;
+// Passes of at most this many roots start with tail rounds.
+constexpr int kTailFirst = 8192;
+// Tail rounds of a batch: most short passes are done after two to six, and an
+// empty one costs 8 us.
+constexpr int kTailRounds = 6;
 
 // The FP64 band re-decision is compiled for soft shadows only; the other
 // applications map it to the float votes (their kernels are not built twice).
@@ -2138,6 +2152,7 @@ struct RoundRunner {
     // (default: a sixth of the trace grid's lanes, about two warps' worth per SM -- the fused kernel clips
     // inside the divergent walk, which only pays once the queue no longer fills the GPU)
     tailRecords = c->cfg.tail_records > 0 ? c->cfg.tail_records : int64_t(gT) * kThreads / 6;
+    p.tailMax = int(std::min<int64_t>(2 * tailRecords, INT_MAX));
     const int yieldPct = c->cfg.yield_pct == 0 ? 50 : std::min(c->cfg.yield_pct, 100);
     yieldAt = yieldPct < 0 ? INT_MAX : std::max(1, int(int64_t(gT) * kWarps * yieldPct / 100));
     static_assert(2 * kRoundsPerCheck <= 32, "kernel_timing events");
@@ -2241,7 +2256,7 @@ struct RoundRunner {
       memcpy(g.grids, grids, sizeof grids);
     }
     CK(cudaGraphLaunch(g.exec, c->stream));
-    for (int k = 0; k < kRoundsPerCheck; ++k, ++round) {
+    for (int k = 0; k < (tail ? kTailRounds : kRoundsPerCheck); ++k, ++round) {
       launches += tail ? 2 : (admit ? 4 : 3);
       if (tail) tailRounds++;
     }
@@ -2249,17 +2264,20 @@ struct RoundRunner {
   }
 
   // The launches of one batch of rounds on the engine's stream
-  // (kFirstRounds at the start of a pass, else kRoundsPerCheck; full rounds:
-  // admit, trace, clip; tail rounds: the fused kernel; then the bookkeeping
-  // kernel), with the kernel_timing events when `events`; returns the rounds.
+  // (kTailRounds tail rounds; full rounds: kFirstRounds at the start of a pass,
+  // else kRoundsPerCheck; full rounds: admit, trace, clip; tail rounds: the
+  // fused kernel; then the bookkeeping kernel), with the kernel_timing events when `events`; returns the rounds.
   // `admit`: some roots are not admitted yet (else the admit kernel, which
   // would find none, is not launched).
   int launchRounds(bool tail, bool admit, bool events) {
     const int n = p.numRoots;
-    const int nr = round == 0 ? kFirstRounds : kRoundsPerCheck;
+    const int nr = tail ? kTailRounds : (round == 0 ? kFirstRounds : kRoundsPerCheck);
     for (int k = 0; k < nr; ++k, ++round) {
       p.cur = round & 1;
       if (tail) {
+        // (a pass that starts with tail rounds: what does not fit now is admitted by the next batch)
+        const bool first = admit && k == 0;
+        if (first) admitKernel<App><<<gA, kThreads, 0, c->stream>>>(p);
         if (events) cudaEventRecord(c->kev[2 * k], c->stream);
         if (mode == kVoteFp64)
           traceKernel<App, true, kVoteFp64F<App>><<<gF, kThreads, kLogSmem, c->stream>>>(p);
@@ -2268,7 +2286,7 @@ struct RoundRunner {
         else
           tailGroupKernel<App><<<gF, kThreads, 0, c->stream>>>(p);
         if (events) cudaEventRecord(c->kev[2 * k + 1], c->stream);
-        launches += 2;
+        launches += first ? 3 : 2;
         tailRounds++;
       } else {
         if (admit) admitKernel<App><<<gA, kThreads, 0, c->stream>>>(p);
@@ -2288,23 +2306,35 @@ struct RoundRunner {
           clipKernel<App><<<gC, kThreads, 0, c->stream>>>(p);
         launches += admit ? 4 : 3;
       }
-      roundEndKernel<<<1, 1, 0, c->stream>>>(c->dCtr, p.cur, n);
+      roundEndKernel<<<1, 1, 0, c->stream>>>(c->dCtr, p.cur, n, tail && mode == kVoteFloat ? p.tailMax : INT_MAX);
     }
     return nr;
   }
+
+  // Whether a pass over n roots starts with tail rounds: with few records a
+  // round lasts as long as its longest walk, which eight lanes take in a third
+  // of the time, and a tail round goes on where a full one stops at each clip.
+  // Up to kTailFirst roots that won on every scene measured (B200, two full
+  // rounds first -> tail rounds at once: room ids 256^2 1.24 -> 0.74 ms, room
+  // 64x48 0.86 -> 0.77, 4801 points 1.62 -> 1.33, building mask 1024^2 3.18 ->
+  // 2.48, meeting room ids of 7500 tiles 20.0 -> 17.5); at 10400 roots whose
+  // queue then grows past 10^5 records it lost 3-6%, with 74000 roots it took
+  // three times as long.
+  bool tailFirst(int n) const { return mode == kVoteFloat && n <= std::min<int64_t>(tailRecords, kTailFirst); }
 
   // One batch of rounds, then the counters.
   int batch() {
     const int n = p.numRoots;
     CK(cudaEventRecord(c->rev[0], c->stream));
     // the mode of this batch of rounds, from the counters of the last one
-    const int64_t queued = hc.count[round & 1];
-    const bool tail = round > 0 && hc.rootNext >= n && queued < tailRecords && c->cfg.tail_records >= 0 &&
-                      (round > kFirstRounds || 2 * queued <= n);
+    const int64_t queued = int64_t(hc.count[0]) + hc.count[1];  // (one of the two is empty)
+    const bool tail = c->cfg.tail_records >= 0 &&
+                      (round == 0 ? tailFirst(n)
+                                  : hc.rootNext >= n && queued < tailRecords && (round > kFirstRounds || 2 * queued <= n));
     // (the legacy default stream, which the allocation-free entry point
     // runs on, cannot be captured)
     const bool admit = hc.rootNext < n;
-    int nr = kRoundsPerCheck;
+    int nr = tail ? kTailRounds : kRoundsPerCheck;
     if (c->cfg.graph_rounds && !ktime && c->stream != nullptr && round > 0) {
       const int e = graphBatch(tail, admit);
       if (e) return e;
@@ -2329,7 +2359,7 @@ struct RoundRunner {
     }
     if (roundLog)
       fprintf(roundLog, "pass %d rounds %d inflight %d rootNext %d/%d queue %d yields %d ms %.3f\n", pass, hc.rounds,
-              hc.inflight, hc.rootNext, n, hc.count[round & 1], hc.yields, ms);
+              hc.inflight, hc.rootNext, n, hc.count[0] + hc.count[1], hc.yields, ms);
     if (hc.error) {
       setErr(hc.error == 2 ? "malformed sub-beam record" : "sub-beam queue overflow (capacity %d)", c->capacity);
       return BT_ERR_CAPACITY;

@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 
 COUNTERS = ["kd_steps", "leaf_visits", "tri_tests", "hits", "splits", "beams", "root_beams", "presplit_beams",
             "five_splits", "climbs"]
-# never tail rounds; tail rounds whenever every root is admitted; records handed on early; the default
-MODES = [dict(tail_records=-1), dict(tail_records=1 << 30), dict(yield_pct=1), {}]
+# never tail rounds; tail rounds throughout; tail rounds that leave a queue grown past 2 x 300 records to full
+# rounds; records handed on early; the default
+MODES = [dict(tail_records=-1), dict(tail_records=1 << 30), dict(tail_records=300), dict(yield_pct=1), {}]
 
 
 def _soup(n=300, seed=5):
@@ -40,7 +41,7 @@ def _counters(info, st):
 
 
 @pytest.mark.parametrize("name", ["room", "plant", "displaced_sphere", "soup"])
-@pytest.mark.parametrize("mode", MODES, ids=["full", "tail", "yield", "default"])
+@pytest.mark.parametrize("mode", MODES, ids=["full", "tail", "tail then full", "yield", "default"])
 def test_pieces_and_counters_equal_emulator(name, mode, gpu):
     from beamtrace2007_b200.renderer import GpuRenderer
     from emu import Emulator
