@@ -10,8 +10,8 @@
 //          per warp for all idle lanes, ballot/popc compaction).  Records
 //          that need a clip go to the bottom of the clip queue, finished
 //          pieces to its top;
-//   clip   one lane per clip record (pieces go to the next round's trace
-//          queue, siblings in consecutive slots) and per finished piece
+//   clip   eight lanes per clip record (pieces go to the next round's trace
+//          queue, siblings in consecutive slots), one lane per finished piece
 //          (the output step: soft-shadow accumulators, polygon lists);
 // plus a one-thread bookkeeping kernel.  Every warp works on every root, so
 // no lane starves while work exists anywhere on the GPU.
@@ -731,12 +731,12 @@ __device__ __forceinline__ void flushStats(const RoundParams& p, const Stats& st
   }
 }
 
-// Each clipping thread's piece log (clipRecord), in dynamic shared memory
-// rather than the thread's local frame: kThreads logs of 10 pieces, 55.8 KB
+// Each clipping thread's piece log in the kernels that clip one record per lane
+// (clipRecord: the logging and FP64 modes), in dynamic shared memory rather
+// than the thread's local frame: kThreads logs of 10 pieces, 55.8 KB
 // a CTA, which still lets 4 clip CTAs share an SM (a log of 8 pieces was
 // 0.5 ms a plant frame slower, one of 6 1.5 ms: the clips it cannot hold
-// are clipped again).  The clip and fused trace kernels are launched with
-// kLogSmem bytes.
+// are clipped again).  These kernels are launched with kLogSmem bytes.
 extern __shared__ PieceLog s_pieceLog[];
 constexpr size_t kLogSmem = sizeof(PieceLog) * kThreads;
 
@@ -1093,9 +1093,17 @@ __global__ void __launch_bounds__(kThreads) admitKernel(const __grid_constant__ 
 // (At least `Ctas` CTAs per SM.  3 lets the compiler keep the lane's state
 // in up to 170 registers; 4 caps it at 128 with a few spills and 16 warps
 // per SM, which pays on a scene that sits in L1/L2 and costs on a larger
-// one (trace_ctas).  The tail-round variant clips inline with its polygons
-// in registers and takes 2 CTAs per SM: tail rounds hold too few records to
-// need more warps.)
+// one (trace_ctas).  The tail-round variant (Fused: the logging and FP64 modes;
+// tailGroupKernel otherwise) clips inline with its polygons in registers and
+// takes 2 CTAs per SM: tail rounds hold too few records to need more warps.)
+//
+// Bound: instruction issue and fetch, with 3-4 lanes at the same kind of step.
+// Tried in its place and slower (B200): four lanes per record, eight records a
+// warp going through their steps together (plant 512^2 18.7 -> 16.9 ms, but
+// meeting room ids 14.9 -> 18.4 and 12 small jobs 69 -> 81: the lines of all
+// edges for every test); a record per lane and each turn the step that most
+// lanes are at (plant 17.2 -> 16.1, but meeting 11.2 -> 15.7, building mask 3.2
+// -> 4.1: 39-49% of issue slots, waiting for instructions).
 template <int App, bool Fused, int Mode = kVoteFloat, int Ctas = 3>
 __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const __grid_constant__ RoundParams p) {
   const int lane = laneId();
