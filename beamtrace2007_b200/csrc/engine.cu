@@ -891,7 +891,7 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
   Line L;
   int flags;
   V3 r0, r1, r2;
-  if (laneCoefs<8, Nearest>(q, t, h, L, flags, r0, r1, r2)) L = makeLine(L.a, L.b, L.c, q.ext);
+  if (laneCoefs<8, Nearest>(q, t, h, L, flags, r0, r1, r2) == kLineCoefs) L = makeLine(L.a, L.b, L.c, q.ext);
   const int nl = !Nearest || h.tri >= 0 ? 4 : 3;
   float newArea;
   int slots0, slots1, count, five;

@@ -72,3 +72,22 @@ def test_pieces_and_counters_equal_emulator(name, mode, gpu):
         assert r.info["retried_roots"] == 0 and _counters(r.info, st) == {}
         # fixed point against double sums of the same pieces, each rounded to float
         assert np.abs(r.vis - vis).max() <= 1e-6 and np.abs(r.E - G).max() <= 1e-6 * max(1.0, np.abs(G).max())
+
+
+@pytest.mark.parametrize("fov, tile", [(179.995, 16), (179.998, 16), (179.9999, 4), (179.9999, 16)])
+def test_views_close_to_180_degrees(fov, tile, gpu):
+    """A root's eps is 2e-5 of its extent on the image plane and passes 1 at an
+    extent of 5e4: a record without a hit has no depth line to be outside of."""
+    from beamtrace2007_b200.renderer import GpuRenderer, make_camera
+    from emu import Emulator
+    s, ps = scene("room")
+    v = s.views[0]
+    cam = make_camera(v.eye, v.target, fov, s.up, 16, 16)
+    pe, st = Emulator(ps).primary_tiles(cam, tile=tile)
+    pe = pe.select(pe.tri >= 0)
+    assert len(pe) > 0
+    for mode in (dict(tail_records=-1), {}):
+        with GpuRenderer(ps, **mode) as g:
+            prim = g.primary(cam, tile=tile)
+            assert np.array_equal(piece_keys(prim, True), piece_keys(pe, True))
+            assert _counters(g.last_info, st) == {}
