@@ -489,7 +489,9 @@ struct AdmitEnv {
 // wavefront_core.h:367-422): the slots pass 1 counted are reserved with one
 // atomic and each piece is written straight into its own, so siblings stay
 // adjacent; slots left by slivers that beamGeom drops are filled with empty
-// records (n = -1), which the trace kernel skips.
+// records (n = 0).  An empty record stays one of its root's live sub-beams
+// until the next round takes it off: a queue then never holds more records
+// than are reserved for, so it cannot overflow.
 template <int App>
 struct SplitEnv {
   const RoundParams* p;
@@ -513,8 +515,8 @@ struct SplitEnv {
     dst = p->tq[nxt] + at;
     reserved = n;
   }
-  // empty records in the slots no piece took; returns their number
-  __device__ int finish() {
+  // empty records in the slots no piece took
+  __device__ void finish() {
     for (int i = filled; i < reserved; ++i) {
       SubBeam d;
       for (int k = 0; k < 4; ++k) d.qx[k] = d.qy[k] = 0.f;
@@ -524,11 +526,10 @@ struct SplitEnv {
       d.hit = -1;
       d.cursor = 0;
       d.depth = 0;
-      d.n = -1;
+      d.n = 0;
       d.neg = 0;
       dst[i] = d;
     }
-    return reserved - filled;
   }
   __device__ bool queue(const SubBeam& r) {
     if (keep && !kept) {
@@ -797,12 +798,12 @@ __device__ __noinline__ bool clipRecord(const RoundParams& p, SubBeam* recp, Sta
   // rest take reserved queue slots
   env.reserve(keep ? slots - 1 : slots);
   splitPass2<SplitEnv<App>, F64>(q, rec, b, ti, L, nl, env, st, &log, e64);
-  // slivers dropped by beamGeom were counted in `slots` but never queued
-  // (nor kept); with no piece at all (slots = 0) there was no kept slot to
-  // give back: the record itself was already taken off by the add above
-  const int unused = env.finish() + (keep && slots > 0 && !env.kept ? 1 : 0);
+  env.finish();
+  // no piece stayed with the lane: its share of `slots` goes back; with no
+  // piece at all (slots = 0) there was none to give back: the record itself
+  // was already taken off by the add above
+  if (keep && slots > 0 && !env.kept) liveSub(p, root, 1);
   if (kept) *kept = env.kept;
-  if (unused > 0) liveSub(p, root, unused);
   return false;
 }
 
@@ -1015,16 +1016,16 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
       }
     }
   }
-  // slivers dropped were counted in `slots` but never queued (nor kept): empty
-  // records (n = -1) in their slots; with no piece at all (slots = 0) there was
-  // no kept slot to give back: the record itself was already taken off above
+  // slivers dropped were counted in `slots` but not queued: empty records in
+  // their slots (SplitEnv); no piece stayed with the group: its share of `slots`
+  // goes back (with slots = 0 there was none: the record itself was already
+  // taken off above)
   if (commit) {
-    const int unused = reserved - filled + (Keep && slots > 0 && !kept ? 1 : 0);
-    o.n = -1;
+    o.n = 0;
     o.hit = -1;
     o.cursor = 0;
     for (; filled < reserved; ++filled) storeRec8(dst + filled, o, 0.f, 0.f);
-    if (lead && unused > 0) liveSub(p, r.root, unused);
+    if (lead && Keep && slots > 0 && !kept) liveSub(p, r.root, 1);
     if (Keep && kept) {
       res = kClipKept;
       v = kv;
@@ -1160,12 +1161,10 @@ __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const 
       const int i = base + __popc(idle & ltMask);
       if (phase == kIdle && i < nCur) {
         r = queue[i];
-        if (uint32_t(r.root) >= uint32_t(p.rootCap) || r.node >= p.s.numNodes || r.n > 4) {
+        if (uint32_t(r.root) >= uint32_t(p.rootCap) || r.node >= p.s.numNodes || r.n < 0 || r.n > 4) {
           atomicExch(&p.ctr->error, 2);  // a malformed record: report, never index with it
-        } else if (r.n < 0) {
-          // an empty slot of a clip's reservation
         } else if (r.n == 0 || p.state[r.root] == kRootKilled) {
-          liveSub(p, r.root, 1);  // a dropped sliver or an abandoned root
+          liveSub(p, r.root, 1);  // an empty slot of a clip's reservation or an abandoned root
         } else {
           if (r.root != qRoot) {
             loadRoot<App>(&p.roots[r.root], q, lightArea);
@@ -1347,12 +1346,10 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
       if (((idle >> W::base()) & 1u) && i < nCur) {
         float4 X, Y;
         loadRec(queue + i, g.r, X, Y);
-        if (uint32_t(g.r.root) >= uint32_t(p.rootCap) || g.r.node >= p.s.numNodes || g.r.n > 4) {
+        if (uint32_t(g.r.root) >= uint32_t(p.rootCap) || g.r.node >= p.s.numNodes || g.r.n < 0 || g.r.n > 4) {
           if (lead) atomicExch(&p.ctr->error, 2);  // a malformed record: report, never index with it
-        } else if (g.r.n < 0) {
-          // an empty slot of a clip's reservation
         } else if (g.r.n == 0 || p.state[g.r.root] == kRootKilled) {
-          if (lead) liveSub(p, g.r.root, 1);  // a dropped sliver or an abandoned root
+          if (lead) liveSub(p, g.r.root, 1);  // an empty slot of a clip's reservation or an abandoned root
         } else {
           if (g.r.root != qRoot) {
             loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);

@@ -91,3 +91,28 @@ def test_views_close_to_180_degrees(fov, tile, gpu):
             prim = g.primary(cam, tile=tile)
             assert np.array_equal(piece_keys(prim, True), piece_keys(pe, True))
             assert _counters(g.last_info, st) == {}
+
+
+@pytest.mark.parametrize("name, size, tile, capacity", [("plant", (45, 33), 16, 5120), ("plant", (45, 33), 16, 6656),
+                                                        ("meeting", (64, 48), 8, 7168)])
+def test_queues_near_their_capacity(name, size, tile, capacity, gpu):
+    """Roots that need about all of a small queue: the pass ends with every
+    piece, or with roots still over budget after the last retry -- never with a
+    queue that holds more records than were reserved for."""
+    from beamtrace2007_b200 import _native
+    from beamtrace2007_b200.renderer import GpuRenderer, make_camera
+    from emu import Emulator
+    s, ps = scene(name)
+    v = s.views[0]
+    cam = make_camera(v.eye, v.target, v.fov, s.up, *size)
+    pe, _ = Emulator(ps).primary_tiles(cam, tile=tile)
+    want = piece_keys(pe.select(pe.tri >= 0), True)
+    for _ in range(3):
+        with GpuRenderer(ps, primary_budget=256, capacity=capacity) as g:
+            try:
+                prim = g.primary(cam, tile=tile)
+            except _native.BtError as e:
+                assert "still over budget" in str(e)
+                continue
+            assert g.last_info["max_spill"] <= capacity
+            assert np.array_equal(piece_keys(prim, True), want)
