@@ -2325,7 +2325,18 @@ struct RoundRunner {
   // 2.48, meeting room ids of 7500 tiles 20.0 -> 17.5); at 10400 roots whose
   // queue then grows past 10^5 records it lost 3-6%, with 74000 roots it took
   // three times as long.
-  bool tailFirst(int n) const { return mode == kVoteFloat && n <= std::min<int64_t>(tailRecords, kTailFirst); }
+  //
+  // A tail round runs each record's chain of splits to its end, which leaves
+  // more sub-beams waiting than full rounds do (plant 45x33, a 16-pixel tile
+  // alone: 7100 at most, 5000 after ten full rounds first).  That only costs
+  // retries while there are any left; but a retried root must not be lost to a
+  // queue that it fits in full rounds.  So a retry pass starts with tail rounds
+  // only where the queue covers every root's whole budget, and the last one
+  // never does.
+  bool tailFirst(int n) const {
+    return mode == kVoteFloat && n <= std::min<int64_t>(tailRecords, kTailFirst) && pass < c->cfg.max_retries &&
+           (pass == 0 || int64_t(n) * p.budget <= c->capacity);
+  }
 
   // One batch of rounds, then the counters.
   int batch() {

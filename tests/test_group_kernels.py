@@ -116,3 +116,18 @@ def test_queues_near_their_capacity(name, size, tile, capacity, gpu):
                 continue
             assert g.last_info["max_spill"] <= capacity
             assert np.array_equal(piece_keys(prim, True), want)
+
+
+def test_retried_root_fits_in_full_rounds(gpu):
+    """One root that a queue holds in full rounds but not with every chain of
+    splits run to its end at once: the retry passes have to find it room."""
+    from beamtrace2007_b200.renderer import GpuRenderer, make_camera
+    from emu import Emulator
+    s, ps = scene("displaced_sphere", subdiv=5)
+    v = s.views[0]
+    cam = make_camera(v.eye, v.target, v.fov, s.up, 45, 33)
+    pe, _ = Emulator(ps).primary_tiles(cam, tile=45)
+    with GpuRenderer(ps, capacity=12288) as g:
+        prim = g.primary(cam, tile=45)
+        assert g.last_info["retried_roots"] > 0
+    assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
