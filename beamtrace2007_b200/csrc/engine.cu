@@ -863,6 +863,15 @@ __device__ __forceinline__ int groupAppend(const RoundParams& p, int q, int n) {
   return n > 0 ? at + before : -1;
 }
 
+// Whether a group's root has been abandoned (`ask`: the group wants to know).
+// Other warps abandon roots meanwhile, and a group's lanes have to go on
+// together: lane 0 reads for all of them.
+__device__ __forceinline__ bool groupRootKilled(const RoundParams& p, bool ask, int root) {
+  int s = kRootNone;
+  if (ask && Grp<8>::sub() == 0) s = p.state[root];
+  return Grp<8>::shfl(s, 0) == kRootKilled;
+}
+
 enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
 
 // Clips the records of a warp's four groups (act: the group has one): the
@@ -1343,22 +1352,30 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
       base = __shfl_sync(kFull, base, 0);
       if (base + ni >= nCur) exhausted = true;
       const int i = base + __popc(idle & before);
+      bool beam = false;
+      float4 X, Y;
       if (((idle >> W::base()) & 1u) && i < nCur) {
-        float4 X, Y;
         loadRec(queue + i, g.r, X, Y);
         if (uint32_t(g.r.root) >= uint32_t(p.rootCap) || g.r.node >= p.s.numNodes || g.r.n < 0 || g.r.n > 4) {
           if (lead) atomicExch(&p.ctr->error, 2);  // a malformed record: report, never index with it
-        } else if (g.r.n == 0 || p.state[g.r.root] == kRootKilled) {
-          if (lead) liveSub(p, g.r.root, 1);  // an empty slot of a clip's reservation or an abandoned root
+        } else if (g.r.n == 0) {
+          if (lead) liveSub(p, g.r.root, 1);  // an empty slot of a clip's reservation
         } else {
-          if (g.r.root != qRoot) {
-            loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);
-            qRoot = g.r.root;
-          }
-          g.cx[0] = X.x, g.cx[1] = X.y, g.cx[2] = X.z, g.cx[3] = X.w;
-          g.cy[0] = Y.x, g.cy[1] = Y.y, g.cy[2] = Y.z, g.cy[3] = Y.w;
-          g.begin(p.s, st);
+          beam = true;
         }
+      }
+      if (groupRootKilled(p, beam, g.r.root)) {
+        if (lead) liveSub(p, g.r.root, 1);
+        beam = false;
+      }
+      if (beam) {
+        if (g.r.root != qRoot) {
+          loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);
+          qRoot = g.r.root;
+        }
+        g.cx[0] = X.x, g.cx[1] = X.y, g.cx[2] = X.z, g.cx[3] = X.w;
+        g.cy[0] = Y.x, g.cy[1] = Y.y, g.cy[2] = Y.z, g.cy[3] = Y.w;
+        g.begin(p.s, st);
       }
       __syncwarp();
       continue;
@@ -1371,7 +1388,7 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
       g.climb(p.s, g.phase == kGClimb, st);
     } else {
       bool act = g.phase == kGClip;
-      if (act && p.state[g.r.root] == kRootKilled) {
+      if (groupRootKilled(p, act, g.r.root)) {
         if (lead) liveSub(p, g.r.root, 1);
         g.phase = kGIdle;
         act = false;
@@ -1482,8 +1499,8 @@ __global__ void __launch_bounds__(kThreads, kClipCtas) clipKernel(const __grid_c
     GroupRec r;
     float4 X, Y;
     loadRec(p.cq + min(i, nClip - 1), r, X, Y);
-    if (p.state[r.root] == kRootKilled) {
-      if (act && W::sub() == 0) liveSub(p, r.root, 1);
+    if (groupRootKilled(p, act, r.root)) {
+      if (W::sub() == 0) liveSub(p, r.root, 1);
       act = false;
     }
     Query q;

@@ -131,3 +131,27 @@ def test_retried_root_fits_in_full_rounds(gpu):
         prim = g.primary(cam, tile=45)
         assert g.last_info["retried_roots"] > 0
     assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
+
+
+@pytest.mark.parametrize("name", ["room", "plant", "displaced_sphere", "soup"])
+@pytest.mark.parametrize("tail_records", [-1, 1 << 30], ids=["full", "tail"])
+def test_abandoned_roots(name, tail_records, gpu):
+    """Budgets that most splitting roots outgrow: records of abandoned roots meet
+    the clip and tail kernels at every place, and their roots come out of the
+    retries whole (the counters hold the abandoned attempts too)."""
+    from beamtrace2007_b200.renderer import GpuRenderer
+    from emu import Emulator
+    ps, cam, point, light = _setup(name)
+    em = Emulator(ps)
+    with GpuRenderer(ps, budget=4, primary_budget=8, tail_records=tail_records) as g:
+        for tile in (3, 16):
+            prim = g.primary(cam, tile=tile)
+            info = g.last_info
+            pe, st = em.primary_tiles(cam, tile=tile)
+            assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
+            assert 0 < info["overflow_roots"] <= info["retried_roots"] and info["passes"] > 1
+            assert (info["tail_rounds"] == 0) == (tail_records < 0)
+            assert [k for i, k in enumerate(COUNTERS) if info[k] < int(st[i])] == []
+        sh = g.point_shadows(cam, prim, point)
+        pe, _ = em.point(cam, point, prim)
+        assert np.array_equal(piece_keys(sh), piece_keys(pe))
