@@ -2174,7 +2174,7 @@ struct RoundRunner {
     // (default: a sixth of the trace grid's lanes, about two warps' worth per SM -- the fused kernel clips
     // inside the divergent walk, which only pays once the queue no longer fills the GPU)
     tailRecords = c->cfg.tail_records > 0 ? c->cfg.tail_records : int64_t(gT) * kThreads / 6;
-    p.tailMax = int(std::min<int64_t>(2 * tailRecords, INT_MAX));
+    p.tailMax = tailRecords >= INT_MAX / 2 ? INT_MAX : int(2 * tailRecords);  // (any int64: no doubling past it)
     const int yieldPct = c->cfg.yield_pct == 0 ? 50 : std::min(c->cfg.yield_pct, 100);
     yieldAt = yieldPct < 0 ? INT_MAX : std::max(1, int(int64_t(gT) * kWarps * yieldPct / 100));
     static_assert(2 * kRoundsPerCheck <= 32, "kernel_timing events");

@@ -155,3 +155,17 @@ def test_abandoned_roots(name, tail_records, gpu):
         sh = g.point_shadows(cam, prim, point)
         pe, _ = em.point(cam, point, prim)
         assert np.array_equal(piece_keys(sh), piece_keys(pe))
+
+
+@pytest.mark.parametrize("tail_records", [(1 << 30) - 1, 1 << 30, 1 << 62, (1 << 63) - 1])
+def test_huge_tail_records(tail_records, gpu):
+    """Any large tail_records means tail rounds always: twice the value may not
+    fit the kernels' int, nor an int64."""
+    from beamtrace2007_b200.renderer import GpuRenderer
+    from emu import Emulator
+    ps, cam, _, _ = _setup("room")
+    pe, st = Emulator(ps).primary_tiles(cam, tile=16)
+    with GpuRenderer(ps, tail_records=tail_records) as g:
+        prim = g.primary(cam, tile=16)
+        assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
+        assert _counters(g.last_info, st) == {} and g.last_info["tail_rounds"] == g.last_info["rounds"] > 0
