@@ -2110,6 +2110,10 @@ int64_t sceneDeviceBytes(const bt_gpu_ctx* c) {
   return int64_t(c->s.numNodes) * (8 + 32 + 4) + c->numRefs * 64 + c->numTris * 32;
 }
 
+// The next retry pass's budget (no more than a queue can ever hold: int
+// arithmetic on live counts stays in range).
+int retryBudget(int budget) { return int(std::min<int64_t>(int64_t(budget) * 16, std::max(budget, 1 << 30))); }
+
 template <int App>
 struct RoundRunner {
   bt_gpu_ctx* c;
@@ -2458,7 +2462,7 @@ int runRoots(bt_gpu_ctx* c, AppParams app, int R, int budget, bt_run_info* info)
     if (nk == 0) break;
     // retry the abandoned roots with a larger budget
     n = nk;
-    budget *= 16;
+    budget = retryBudget(budget);
   }
   rr.finish(R);
   return BT_OK;
@@ -3842,7 +3846,7 @@ int laneSoftRun(bt_gpu_ctx* c, SoftFeed& feed, double foldMs, bt_run_info* info)
     if ((e = rr.endPass(n, &list, &nk))) return failAll(e);
     if (nk == 0) break;
     n = nk;
-    budget *= 16;
+    budget = retryBudget(budget);
     if ((e = rr.startPass(n, list, budget))) return failAll(e);
     do {
       if ((e = rr.batch())) return failAll(e);

@@ -169,3 +169,17 @@ def test_huge_tail_records(tail_records, gpu):
         prim = g.primary(cam, tile=16)
         assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
         assert _counters(g.last_info, st) == {} and g.last_info["tail_rounds"] == g.last_info["rounds"] > 0
+
+
+def test_retries_of_a_large_budget(gpu):
+    """16 times a budget of 2^20, four times over, is past an int."""
+    from beamtrace2007_b200.renderer import GpuRenderer, make_camera
+    from emu import Emulator
+    s, ps = scene("plant")
+    v = s.views[0]
+    cam = make_camera(v.eye, v.target, v.fov, s.up, 45, 33)
+    pe, _ = Emulator(ps).primary_tiles(cam, tile=3)
+    with GpuRenderer(ps, primary_budget=1 << 20, capacity=4096) as g:
+        prim = g.primary(cam, tile=3)
+        assert g.last_info["passes"] > 3
+    assert np.array_equal(piece_keys(prim, True), piece_keys(pe.select(pe.tri >= 0), True))
