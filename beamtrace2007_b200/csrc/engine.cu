@@ -831,7 +831,7 @@ __device__ __forceinline__ void loadRec(const SubBeam* at, GroupRec& r, float4& 
 
 // Writes a record whose corner k lies in lane k of the group (8 lanes, 64 bytes at once).
 __device__ __forceinline__ void storeRec8(SubBeam* at, const GroupRec& r, float x, float y) {
-  const int sub = Grp<8>::sub();
+  const int sub = Grp::sub();
   if (sub < 4) {
     reinterpret_cast<float*>(at)[sub] = x;
     reinterpret_cast<float*>(at)[4 + sub] = y;
@@ -844,7 +844,7 @@ __device__ __forceinline__ void storeRec8(SubBeam* at, const GroupRec& r, float 
 // group's lanes) with one atomic; returns the group's first slot, or -1 (and
 // flags an error) if they do not fit, which the reservation rule rules out.
 __device__ __forceinline__ int groupAppend(const RoundParams& p, int q, int n) {
-  using W = Grp<8>;
+  using W = Grp;
   int before = 0, total = 0;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
@@ -868,8 +868,8 @@ __device__ __forceinline__ int groupAppend(const RoundParams& p, int q, int n) {
 // together: lane 0 reads for all of them.
 __device__ __forceinline__ bool groupRootKilled(const RoundParams& p, bool ask, int root) {
   int s = kRootNone;
-  if (ask && Grp<8>::sub() == 0) s = p.state[root];
-  return Grp<8>::shfl(s, 0) == kRootKilled;
+  if (ask && Grp::sub() == 0) s = p.state[root];
+  return Grp::shfl(s, 0) == kRootKilled;
 }
 
 enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
@@ -886,7 +886,7 @@ enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
 template <int App, bool Keep>
 __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, bool act, GroupRec& r, LanePoly& v,
                                           const Query& q, float lightArea, const HitPlane& h, Stats& st) {
-  using W = Grp<8>;
+  using W = Grp;
   constexpr bool Nearest = App == kAppPrimary;
   const int sub = W::sub();
   const bool lead = sub == 0;
@@ -901,7 +901,7 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
   Line L;
   int flags;
   V3 r0, r1, r2;
-  if (laneCoefs<8, Nearest>(q, t, h, L, flags, r0, r1, r2) == kLineCoefs) L = makeLine(L.a, L.b, L.c, q.ext);
+  if (laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2) == kLineCoefs) L = makeLine(L.a, L.b, L.c, q.ext);
   const int nl = !Nearest || h.tri >= 0 ? 4 : 3;
   float newArea;
   int slots0, slots1, count, five;
@@ -1292,10 +1292,9 @@ __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const 
 template <int App>
 __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __grid_constant__ RoundParams p) {
   __shared__ ClipScratch scratch[kThreads / 8];
-  constexpr int G = 8;
   constexpr bool Nearest = App == kAppPrimary;
   constexpr unsigned kLeads = 0x01010101u;
-  using W = Grp<G>;
+  using W = Grp;
   const int lane = laneId(), sub = W::sub();
   const bool lead = sub == 0;
   const unsigned before = (1u << W::base()) - 1u;
@@ -1305,8 +1304,8 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
   bool exhausted = nCur == 0;
   // few records: spread over the warps, so that a warp's groups do not wait for each other's steps
   const int warps = gridDim.x * kWarps;
-  const int most = max(1, min(32 / G, (nCur + warps - 1) / warps));
-  GroupWalk<G, Nearest> g;
+  const int most = max(1, min(4, (nCur + warps - 1) / warps));
+  GroupWalk<Nearest> g;
   g.idle();
   float lightArea = 0.f;
   int qRoot = -1;
@@ -1482,7 +1481,7 @@ __device__ __forceinline__ bool clipQueueFits(const RoundParams& p, int nClip, i
 template <int App>
 __global__ void __launch_bounds__(kThreads, kClipCtas) clipKernel(const __grid_constant__ RoundParams p) {
   __shared__ ClipScratch scratch[kThreads / 8];
-  using W = Grp<8>;
+  using W = Grp;
   const int lane = laneId();
   const int nClip = p.ctr->clipCount, nOut = p.ctr->outQ;
   if (!clipQueueFits(p, nClip, nOut)) return;
@@ -2099,10 +2098,11 @@ constexpr int kTailFirst = 8192;
 // empty one costs 8 us.
 constexpr int kTailRounds = 6;
 
-// The FP64 band re-decision is compiled for soft shadows only; the other
-// applications map it to the float votes (their kernels are not built twice).
+// The FP64 band re-decision is compiled for soft shadows only.  The launches of
+// the other applications, which never run in that mode, name their logging
+// kernels, so that no further kernel is built for them.
 template <int App>
-constexpr int kVoteFp64F = App == kAppSoft ? kVoteFp64 : kVoteFloat;
+constexpr int kVoteFp64F = App == kAppSoft ? kVoteFp64 : kVoteLog;
 
 // The resident scene pool's bytes on the device: kd nodes and boxes, leaf
 // references, triangle normals and planes.

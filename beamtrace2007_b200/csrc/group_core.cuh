@@ -23,18 +23,18 @@ namespace btg {
 
 // --------------------------------------------------------- lanes of a group
 
-template <int G>
+// A group: eight lanes side by side, four groups a warp.
 struct Grp {
   static __device__ __forceinline__ int lane() { return threadIdx.x & 31; }
-  static __device__ __forceinline__ int sub() { return threadIdx.x & (G - 1); }
-  static __device__ __forceinline__ int base() { return threadIdx.x & 31 & ~(G - 1); }
+  static __device__ __forceinline__ int sub() { return threadIdx.x & 7; }
+  static __device__ __forceinline__ int base() { return threadIdx.x & 24; }
   // the group's lanes for which `pred` holds, bit 0 = its first lane
   static __device__ __forceinline__ unsigned ballot(bool pred) {
-    return (__ballot_sync(0xffffffffu, pred) >> base()) & (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u);
+    return (__ballot_sync(0xffffffffu, pred) >> base()) & 0xffu;
   }
   template <class T>
   static __device__ __forceinline__ T shfl(T v, int src) {
-    return __shfl_sync(0xffffffffu, v, src, G);
+    return __shfl_sync(0xffffffffu, v, src, 8);
   }
 };
 
@@ -60,7 +60,7 @@ enum LaneLine { kLineNone = 0, kLineConst = 1, kLineCoefs = 2 };
 // Edge lines and the depth line of triangle t, one per lane, before they are
 // normalised (BeamCtx::triSetup and closerLine, as testOne evaluates them).
 // `flags`: kTriPlain | kTriFront, the same in all lanes of the group.
-template <int G, bool Nearest>
+template <bool Nearest>
 __device__ __forceinline__ LaneLine laneCoefs(const Query& q, const TriRec& t, const HitPlane& h, Line& L,
                                               int& flags, V3& r0, V3& r1, V3& r2) {
   const int e = threadIdx.x & 3;
@@ -77,7 +77,7 @@ __device__ __forceinline__ LaneLine laneCoefs(const Query& q, const TriRec& t, c
     if (notEdgeOn(D, m, r2)) fl |= kTriPlain;
     if (D > 0) fl |= kTriFront;
   }
-  flags = Grp<G>::shfl(fl, 0);
+  flags = Grp::shfl(fl, 0);
   if (e == 3) m = t.n;
   L.a = dot(m, q.P.u);
   L.b = dot(m, q.P.v);
@@ -126,14 +126,13 @@ enum GroupPhase {
   kGClip = 5      // the triangle at the cursor needs a clip
 };
 
-// A record being walked by a group of G lanes (4 or 8; lane k and lane k + 4
-// hold corner k & 3).  The steps are those of engine_core.cuh (descendStep,
+// A record being walked by a group (lane k and lane k + 4 hold corner k & 3).  The steps are those of engine_core.cuh (descendStep,
 // climbStep, testOne) with the four corners, and the up to four lines of a
 // triangle, side by side; a step's corner comparisons are packed into one word
 // and the lanes' words combined by two shuffles.
-template <int G, bool Nearest>
+template <bool Nearest>
 struct GroupWalk {
-  using W = Grp<G>;
+  using W = Grp;
   GroupRec r;
   Query q;
   float cx[4], cy[4];  // every corner (the lines' votes)
@@ -343,7 +342,7 @@ struct GroupWalk {
     Line L;
     int flags;
     V3 r0, r1, r2;
-    const LaneLine line = laneCoefs<G, Nearest>(q, t, h, L, flags, r0, r1, r2);
+    const LaneLine line = laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2);
     bool anyIn = line == kLineNone || L.c > q.eps, anyOut = L.c < -q.eps;  // (a constant line's vote)
     const bool known = line != kLineCoefs || voteUnscaled(cx, cy, L.a, L.b, L.c, max4abs(cx), max4abs(cy), q.eps, q.ext,
                                                           anyIn, anyOut);
@@ -361,7 +360,7 @@ struct GroupWalk {
     }
     const unsigned in = W::ballot(anyIn), out = W::ballot(anyOut);
     const bool counted = act && t.tri != q.exclude && (flags & kTriPlain) && !(Nearest && q.cull && (flags & kTriFront));
-    const bool meets = counted && !(Nearest && h.tri == t.tri) && in == (1u << G) - 1u;
+    const bool meets = counted && !(Nearest && h.tri == t.tri) && in == 0xffu;
     if (counted) st.triTests++;
     const bool inside = meets && out == 0;
     bool clip = meets && out != 0;
@@ -404,7 +403,7 @@ struct GroupWalk {
 
 // Signed area (Poly::area): the terms are summed in vertex order.
 __device__ __forceinline__ float groupArea(float px, float py, int n) {
-  using W = Grp<8>;
+  using W = Grp;
   const int nx = W::sub() + 1 == n ? 0 : W::sub() + 1;
   const float xn = W::shfl(px, nx), yn = W::shfl(py, nx);
   const float t = px * yn - xn * py;
@@ -436,7 +435,7 @@ __device__ __forceinline__ void cleanBegin(CleanState& s, const LanePoly& p, boo
   s.i0 = 0;
 }
 __device__ __forceinline__ void cleanStep(CleanState& s, LanePoly& p, float eps) {
-  using W = Grp<8>;
+  using W = Grp;
   const int sub = W::sub();
   const int h = sub == 0 ? p.n - 1 : sub - 1, j = sub + 1 >= p.n ? 0 : sub + 1;
   const float xh = W::shfl(p.x, h), yh = W::shfl(p.y, h), xj = W::shfl(p.x, j), yj = W::shfl(p.y, j);
@@ -516,7 +515,7 @@ struct __align__(16) ClipScratch {
 // split inside the clip.
 __device__ __forceinline__ bool groupClip(float eps, LanePoly p, const Line& L, int nl, bool act, ClipScratch& S,
                                           float& newArea, int& slots0, int& slots1, int& count, int& five) {
-  using W = Grp<8>;
+  using W = Grp;
   const int sub = W::sub();
   const unsigned lt = (1u << sub) - 1u;
   newArea = 0.f;
