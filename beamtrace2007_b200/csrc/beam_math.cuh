@@ -264,14 +264,10 @@ BT_HD Line makeLine(float a, float b, float c, float ext) {
 // three edges, and the line out of line (B200): plant 512^2 17.7 -> 17.2 ms,
 // 333x217 at light scale 4 42.5 -> 41.1, 12 small jobs 71.2 -> 68.7, room 64x48
 // 0.91 -> 0.86.
-BT_HD bool voteUnscaled(const float* qx, const float* qy, float a, float b, float c, float maxX, float maxY, float eps,
-                        float ext, bool& in, bool& out) {
-  const float nn = a * a + b * b;
-#if defined(__CUDA_ARCH__)
-  const float nrm = nn * rsqrtf(nn);
-#else
-  const float nrm = std::sqrt(nn);
-#endif
+//
+// (voteUnscaledNorm takes nn = a a + b b and the approximate norm.)
+BT_HD bool voteUnscaledNorm(const float* qx, const float* qy, float a, float b, float c, float nn, float nrm, float maxX,
+                            float maxY, float eps, float ext, bool& in, bool& out) {
   const float T = eps * nrm, ac = fabs_(c);
   if (!(nn > 1e-24f && nn < 1e24f && T > 1e-24f && nrm * ext * 0.9e9f > ac && ac < 1e24f)) return false;
   const float S = maxX * fabs_(a) + maxY * fabs_(b) + ac;
@@ -286,6 +282,16 @@ BT_HD bool voteUnscaled(const float* qx, const float* qy, float a, float b, floa
   in = hi > T;
   out = lo < -T;
   return true;
+}
+BT_HD bool voteUnscaled(const float* qx, const float* qy, float a, float b, float c, float maxX, float maxY, float eps,
+                        float ext, bool& in, bool& out) {
+  const float nn = a * a + b * b;
+#if defined(__CUDA_ARCH__)
+  const float nrm = nn * rsqrtf(nn);  // (2 ulp by the CUDA C++ Programming Guide's error table, 1/2 for the product)
+#else
+  const float nrm = std::sqrt(nn);
+#endif
+  return voteUnscaledNorm(qx, qy, a, b, c, nn, nrm, maxX, maxY, eps, ext, in, out);
 }
 
 // An edge line in FP64 (the opt-in band re-decision, eps_fp64): the same

@@ -4,7 +4,9 @@
 // root sequentially: admission, trace to the next clip, two-pass clip, with a
 // FIFO of records instead of the GPU's warps and queues.  The pieces it
 // produces must equal the reference BeamCore's (trail, no mailbox) bit for
-// bit; the CUDA kernels run the same functions per lane.
+// bit; the CUDA kernels run the same functions per lane, except that triangles
+// are tested here by their normalised lines (testByLine), not by the unscaled
+// votes of testOne, which runs beside it and is counted where it differs.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -80,6 +82,58 @@ struct RootEnv {
   void dropped(float) {}
 };
 
+// Tests the pending triangle as BeamCtx::classifyTri is written
+// (beam_core.h:376-408): the full triangle setup, then every corner's distance
+// to the normalised lines.
+int testByLine(const SceneDev& s, const Query& q, SubBeam& r, Beam& B, Stats& st, int& occluder) {
+  const TriRec t = loadRef(s, s.node[r.node].x + uint32_t(r.cursor));
+  r.cursor += 1;
+  TriInfo ti;
+  triSetup(q, t.v0, t.v1, t.v2, t.n, t.vi, t.tri, ti);
+  if (!ti.ok) return kStepContinue;
+  st.triTests++;
+  if (B.hit == t.tri) return kStepContinue;
+  bool allIn = true;
+  for (int k = 0; k < 3; ++k)
+    if (!voteLine(q, B, ti.edge[k], allIn)) return kStepContinue;
+  if (q.mode == kModeNearest && B.hit >= 0 &&
+      !voteLine(q, B, closerLine(q, ti, B.hitA, B.hitC, B.hitN, B.hit), allIn))
+    return kStepContinue;
+  const float farA[3] = {0.f, 0.f, q.farCq};
+  if (q.farIsPlane && !voteLine(q, B, closerLine(q, ti, farA, q.farCq, q.P.n, -1), allIn)) return kStepContinue;
+  if (!allIn) {
+    if (separated(q, B, ti)) return kStepContinue;
+    r.cursor -= 1;
+    return kStepSplit;
+  }
+  if (q.mode == kModeAnyHit) {
+    occluder = t.tri;
+    return kStepFinished;
+  }
+  setStatus(q, B, t.tri, ti.A, ti.C);
+  for (int k = 0; k < 3; ++k) B.hitA[k] = ti.A[k];
+  B.hitC = ti.C;
+  B.hitN = ti.n;
+  r.hit = t.tri;
+  return kStepContinue;
+}
+
+// testByLine, with testOne beside it on copies.
+uint64_t testsRun = 0, testsDiffer = 0;
+int testBoth(const SceneDev& s, const Query& q, SubBeam& r, Beam& B, Stats& st, int& occluder) {
+  SubBeam r1 = r;
+  Beam B1 = B;
+  Stats st1 = st;
+  int occ1 = occluder;
+  const int res1 = testOne(s, q, r1, B1, st1, occ1);
+  const int res = testByLine(s, q, r, B, st, occluder);
+  ++testsRun;
+  if (res != res1 || occluder != occ1 || r.cursor != r1.cursor || r.hit != r1.hit || B.hit != B1.hit ||
+      st.triTests != st1.triTests)
+    ++testsDiffer;
+  return res;
+}
+
 // Traces one root to completion; appends all output pieces.
 void traceRoot(const SceneDev& s, const Query& q, const Poly<8>& poly, std::vector<Piece>& out, Stats& st) {
   std::deque<SubBeam> fifo;
@@ -102,7 +156,7 @@ void traceRoot(const SceneDev& s, const Query& q, const Poly<8>& poly, std::vect
       int occ = -1;
       if (res == kStepContinue) {
         for (;;) {
-          res = testOne(s, q, r, b, st, occ);
+          res = testBoth(s, q, r, b, st, occ);
           if (res != kStepContinue || !moreInLeaf(s, q, r)) break;
         }
       }
@@ -534,10 +588,18 @@ EMU_API int emu_decide(const float* O, const float* p0, const float* u, const fl
   return decide(q, b, axis, Ns, box);
 }
 
+// Triangle tests so far, and those in which testOne and testByLine differ.
+EMU_API void emu_tests(uint64_t* out) {
+  out[0] = testsRun;
+  out[1] = testsDiffer;
+}
+
 // The votes of four corners on the line makeLine(a, b, c, ext): out[0], out[1]
 // some corner above eps / below -eps by the line itself, and, if voteUnscaled
-// can tell (the result), out[2], out[3] what it says.  For the vote fuzz test.
-EMU_API int emu_vote(const float* qx, const float* qy, float a, float b, float c, float eps, float ext, int* out) {
+// can tell with a norm that is off by the share `off` of itself (the result),
+// out[2], out[3] what it says.  For the vote fuzz test.
+EMU_API int emu_vote(const float* qx, const float* qy, float a, float b, float c, float eps, float ext, double off,
+                     int* out) {
   const Line L = makeLine(a, b, c, ext);
   out[0] = out[1] = 0;
   for (int k = 0; k < 4; ++k) {
@@ -546,7 +608,9 @@ EMU_API int emu_vote(const float* qx, const float* qy, float a, float b, float c
     out[1] |= dv < -eps;
   }
   bool in = false, below = false;
-  const int known = voteUnscaled(qx, qy, a, b, c, max4abs(qx), max4abs(qy), eps, ext, in, below);
+  const float nn = a * a + b * b;
+  const int known = voteUnscaledNorm(qx, qy, a, b, c, nn, float(double(std::sqrt(nn)) * (1 + off)), max4abs(qx),
+                                     max4abs(qy), eps, ext, in, below);
   out[2] = in;
   out[3] = below;
   return known;

@@ -36,6 +36,12 @@ class Emulator:
         except Exception:
             pass
 
+    def tests(self):
+        """Triangle tests of all emulators so far, and those that testOne answers differently."""
+        out = np.zeros(2, np.uint64)
+        self.lib.emu_tests(_p(out))
+        return int(out[0]), int(out[1])
+
     def soft_points(self, light, offset, tri, X, N_, exact=False):
         tri = np.ascontiguousarray(tri, np.int32)
         X = np.ascontiguousarray(X, np.float32)
