@@ -16,10 +16,11 @@
 // plus a one-thread bookkeeping kernel.  Every warp works on every root, so
 // no lane starves while work exists anywhere on the GPU.
 //
-// Memory is bounded without waiting: a root is admitted only if `budget`
-// queue slots are free for it, and a root that would exceed its budget is
-// abandoned and traced again, on the GPU, in a retry pass with a 16x budget
-// (the reference recomputed such roots on the CPU, cuda/gpu_render.cu:651-672).
+// Memory is bounded without waiting: a root is admitted only if its first queue
+// slots are free (at most 128, kInitialReserve), takes more as it grows, and a
+// root that would exceed its budget, or the queues' free slots, is abandoned
+// and traced again, on the GPU, in a retry pass with a 16x budget (the reference
+// recomputed such roots on the CPU, cuda/gpu_render.cu:651-672).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -63,6 +64,13 @@ void setErr(const char* fmt, ...) {
   } while (0)
 
 constexpr unsigned kFull = 0xffffffffu;
+// CTAs per SM of the lane-group kernels, i.e. their register caps.  Measured
+// (B200, two runs each, within 1%): clip with 4, 5, 6 and 8 -- plant 512^2 16.57,
+// 16.64, 16.30, 16.42 ms; 333x217 at light scale 4 41.4, 41.3, 40.3, 40.6; meeting
+// room ids and small calls alike.  Tail with 2, 3, 4 and 5 -- 4801 points 1.41,
+// 1.41, 1.39, 1.51 ms; room ids 256^2 0.71, 0.72, 0.75, 0.79; meeting room ids
+// 10.8, 10.8, 11.0, 11.5; polygons 511x389 2.02, 2.02, 2.08, 2.16: 4 is best for
+// soft shadows only, where rounds hold the most records.
 constexpr int kClipCtas = 6;
 constexpr int kTailCtas = 4;  // (128 registers)
 constexpr int kWarps = 4;
@@ -1107,13 +1115,10 @@ __global__ void __launch_bounds__(kThreads) admitKernel(const __grid_constant__ 
 // tailGroupKernel otherwise) clips inline with its polygons in registers and
 // takes 2 CTAs per SM: tail rounds hold too few records to need more warps.)
 //
-// Bound: instruction issue and fetch, with 3-4 lanes at the same kind of step.
-// Tried in its place and slower (B200): four lanes per record, eight records a
-// warp going through their steps together (plant 512^2 18.7 -> 16.9 ms, but
-// meeting room ids 14.9 -> 18.4 and 12 small jobs 69 -> 81: the lines of all
-// edges for every test); a record per lane and each turn the step that most
-// lanes are at (plant 17.2 -> 16.1, but meeting 11.2 -> 15.7, building mask 3.2
-// -> 4.1: 39-49% of issue slots, waiting for instructions).
+// Bound: instruction issue.  A lane follows its own beam through the tree, so
+// 3.7 of 32 lanes share an instruction; 62% of the issue slots are taken at 16
+// warps per SM, fixed latencies the top stall (a heavy round of the plant,
+// 333x217 at light scale 4: 1.17 ms, 33 GB/s of DRAM).
 template <int App, bool Fused, int Mode = kVoteFloat, int Ctas = 3>
 __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const __grid_constant__ RoundParams p) {
   const int lane = laneId();
@@ -1282,9 +1287,12 @@ __global__ void __launch_bounds__(kThreads, Fused ? 2 : Ctas) traceKernel(const 
 // advances many levels per round.  A warp's four groups go through their steps
 // together, each time the step that most of them are at.
 //
-// Bound: the longest chain of walks and clips, one after the other.  With one
-// lane per record a step loops over four corners and three edges and a clip
-// over six vertices; here they lie side by side, which makes a step about a
+// Bound: the longest chain of walks and clips, one after the other; while many
+// records are left, instruction fetch (the first round of 4801 points on the
+// plant: no_instruction the top stall, 3.5 cycles an issue, 24 of 32 lanes; of
+// room ids 256^2, 256 records: 0.7 warps a scheduler, 20% of the issue slots).
+// With one lane per record a step loops over four corners and three edges and a
+// clip over six vertices; here they lie side by side, which makes a step about a
 // third as long and a clip a tenth.  Tail rounds of a call, one lane -> eight
 // per record (B200): plant 512^2 3.0 -> 1.0 ms, meeting room ids 1024^2 7.2 ->
 // 4.5, 4801 points on the plant 3.4 -> 1.0, two retried roots of the displaced
@@ -1474,7 +1482,9 @@ __device__ __forceinline__ bool clipQueueFits(const RoundParams& p, int nClip, i
 // vertex each: classifying, splitting and cleaning it are a few ballots and
 // shuffles, where one lane per clip unrolled every polygon step six times
 // behind selects (128 registers with spills, 8 of 32 lanes active, instruction
-// fetch its top stall).  73 registers, 25 KB of shared memory a CTA.  Frames,
+// fetch its top stall).  71 registers for soft shadows, 72 for primary beams, 80
+// with 276 bytes of spill stores for point shadows (their occluded pieces are
+// output in the clip); 25.9 KB of shared memory a CTA.  Frames,
 // one lane -> eight lanes per clip (B200): plant 512^2 21.8 -> 18.7 ms, plant
 // 333x217 at light scale 4 49.3 -> 42.1, displaced sphere 512^2 at scale 2
 // 66.8 -> 60.2, meeting room ids at 1024^2 16.8 -> 14.9.
@@ -2080,10 +2090,10 @@ void fillInfo(bt_gpu_ctx* c, const Counters& hc, bt_run_info* info) {
 // Runs every root of `R` through the engine.  A round is three kernels --
 // admit (new roots, as far as the queue reservation allows), trace (drain
 // the round's queue), clip (pieces into the next round's queue) -- plus the
-// bookkeeping kernel; rounds are launched in batches of kRoundsPerCheck
-// between reads of the completion flag (rounds after completion return at
-// once).  Roots abandoned over budget are retried in a further pass with a
-// 16x budget.
+// bookkeeping kernel; rounds are launched in batches of kRoundsPerCheck (tail
+// rounds: kTailRounds) between reads of the completion flag (rounds after
+// completion return at once).  Roots abandoned over budget are retried in a
+// further pass with a 16x budget.
 constexpr int kRoundsPerCheck = 8;
 // Scenes up to this many bytes on the device (kd nodes and boxes, leaf
 // references, triangle normals) take the 4-CTA round trace kernel.
@@ -2175,8 +2185,9 @@ struct RoundRunner {
          : mode == kVoteLog ? gridFor(c, traceKernel<App, true, kVoteLog>, kLogSmem)
                             : gridFor(c, tailGroupKernel<App>);
     // tail rounds: every root admitted and fewer queued records than this
-    // (default: a sixth of the trace grid's lanes, about two warps' worth per SM -- the fused kernel clips
-    // inside the divergent walk, which only pays once the queue no longer fills the GPU)
+    // (default: a sixth of the trace grid's lanes, about two warps' worth per SM: a full queue is worked off
+    // faster a record per lane, a short one, where only the longest chain counts, eight lanes per record;
+    // thresholds from 20000 to 160000 gained nothing)
     tailRecords = c->cfg.tail_records > 0 ? c->cfg.tail_records : int64_t(gT) * kThreads / 6;
     p.tailMax = tailRecords >= INT_MAX / 2 ? INT_MAX : int(2 * tailRecords);  // (any int64: no doubling past it)
     const int yieldPct = c->cfg.yield_pct == 0 ? 50 : std::min(c->cfg.yield_pct, 100);
@@ -2231,7 +2242,8 @@ struct RoundRunner {
     return BT_OK;
   }
 
-  // One batch of kRoundsPerCheck rounds (not the first) as one CUDA graph (graph_rounds):
+  // One batch of rounds (not the first; kTailRounds tail or kRoundsPerCheck full
+  // ones) as one CUDA graph (graph_rounds):
   // the launches are captured once and replayed while their parameters stay
   // the same (a new frame with the same camera, light and buffers replays
   // the graph of the last one); otherwise captured again and the
@@ -2290,9 +2302,10 @@ struct RoundRunner {
   }
 
   // The launches of one batch of rounds on the engine's stream
-  // (kTailRounds tail rounds; full rounds: kFirstRounds at the start of a pass,
-  // else kRoundsPerCheck; full rounds: admit, trace, clip; tail rounds: the
-  // fused kernel; then the bookkeeping kernel), with the kernel_timing events when `events`; returns the rounds.
+  // (kTailRounds tail rounds, or full ones: kFirstRounds at the start of a pass,
+  // else kRoundsPerCheck; a full round: admit, trace, clip; a tail round: the
+  // fused kernel; then the bookkeeping kernel), with the kernel_timing events
+  // when `events`; returns the rounds.
   // `admit`: some roots are not admitted yet (else the admit kernel, which
   // would find none, is not launched).
   int launchRounds(bool tail, bool admit, bool events) {

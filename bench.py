@@ -622,7 +622,8 @@ def main():
                          "benchmark's workload)"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "traceKernel<soft>",
+                         "kernel": "trace launches of a frame: traceKernel<soft>, in tail rounds tailGroupKernel<soft> "
+                                   "(traffic: traceKernel<soft>, three heavy rounds)",
                          "algorithmic_bytes_per_launch": b_trace / launches_per_frame,
                          "launches_per_frame": launches_per_frame,
                          "kernel_ms_per_launch": trace_ms / launches_per_frame,

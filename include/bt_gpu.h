@@ -123,7 +123,9 @@ typedef struct {
   int32_t max_retries;      /* budget x16 retries before BT_ERR_CAPACITY */
   int64_t tail_records;     /* tail rounds (one fused trace-and-clip kernel) below this many queued
                                records once every root is admitted, and from the start for passes over at
-                               most this many and 8192 roots; 0 = a sixth of the trace grid's lanes, < 0 = never */
+                               most this many and 8192 roots (not the last retry pass, nor one whose roots'
+                               budgets the queue does not cover); 0 = a sixth of the trace grid's lanes,
+                               < 0 = never */
   int32_t eps_stats;        /* nonzero: trace kernels that also count the edge votes in the fuzzy band
                                and their FP64 re-evaluation (eps_band_corners, eps_fp64_flips); results
                                are the same, the kernels are slower */
