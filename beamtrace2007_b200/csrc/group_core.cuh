@@ -126,7 +126,8 @@ enum GroupPhase {
   kGClip = 5      // the triangle at the cursor needs a clip
 };
 
-// A record being walked by a group (lane k and lane k + 4 hold corner k & 3).  The steps are those of engine_core.cuh (descendStep,
+// A record being walked by a group (lane k and lane k + 4 hold corner k & 3).
+// The steps are those of engine_core.cuh (descendStep,
 // climbStep, testOne) with the four corners, and the up to four lines of a
 // triangle, side by side; a step's corner comparisons are packed into one word
 // and the lanes' words combined by two shuffles.
