@@ -871,14 +871,14 @@ __device__ __forceinline__ int groupAppend(const RoundParams& p, int q, int n) {
   return n > 0 ? at + before : -1;
 }
 
-// Whether a group's root has been abandoned (`ask`: the group wants to know).
-// Other warps abandon roots meanwhile, and a group's lanes have to go on
-// together: lane 0 reads for all of them.
-__device__ __forceinline__ bool groupRootKilled(const RoundParams& p, bool ask, int root) {
-  int s = kRootNone;
-  if (ask && Grp::sub() == 0) s = p.state[root];
-  return Grp::shfl(s, 0) == kRootKilled;
+// The state of a group's root, read by lane 0 for all of them (`ask`: the group
+// wants to know): other warps abandon roots meanwhile, and a group's lanes have
+// to go on together.  The caller loads what it needs next, then groupKilled
+// tells the group, or lane 0 acts on it alone.
+__device__ __forceinline__ int leadState(const RoundParams& p, bool ask, int root) {
+  return ask && Grp::sub() == 0 ? p.state[root] : int(kRootNone);
 }
+__device__ __forceinline__ bool groupKilled(int leadState) { return Grp::shfl(leadState, 0) == kRootKilled; }
 
 enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
 
@@ -886,7 +886,9 @@ enum { kClipGone = 0, kClipUnchanged = 1, kClipKept = 2 };
 // triangle at a record's cursor needs it.  Pieces go to the next round's trace
 // queue in consecutive slots; with Keep the first piece stays with the group
 // (r and v become it: kClipKept).  kClipUnchanged: nothing measurable changed
-// and the record goes on at its next triangle (r.cursor moved).
+// and the record goes on at its next triangle (r.cursor moved).  The record of a
+// root abandoned before is dropped where it would split (asking first took 2% of
+// a small primary call: one more read and shuffle before the triangle's loads).
 // v: corner k in lane k (lanes past n - 1 repeat the last).
 //
 // Pass 1 (groupClip) logs the pieces and measures what changes status
@@ -902,6 +904,7 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
   t.v0 = t.v1 = t.v2 = t.n = mk(0, 0, 0);
   t.vi[0] = t.vi[1] = t.vi[2] = 0;
   t.tri = -1;
+  const int state = leadState(p, act, r.root);
   if (act) {
     const uint2 leaf = p.s.node[r.node];
     t = loadRef(p.s, leaf.x + uint32_t(r.cursor));
@@ -909,7 +912,7 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
   Line L;
   int flags;
   V3 r0, r1, r2;
-  if (laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2) == kLineCoefs) L = makeLine(L.a, L.b, L.c, q.ext);
+  if (laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2)) L = makeLine(L.a, L.b, L.c, q.ext);
   const int nl = !Nearest || h.tri >= 0 ? 4 : 3;
   float newArea;
   int slots0, slots1, count, five;
@@ -926,7 +929,10 @@ __device__ __forceinline__ int clipGroups(const RoundParams& p, ClipScratch& S, 
   }
   const int slots = slots0 + (Nearest ? slots1 : 0);
   int fits = 1;
-  if (lead && commit) {
+  if (lead && commit && state == kRootKilled) {
+    liveSub(p, r.root, 1);
+    fits = 0;
+  } else if (lead && commit) {
     const int old = atomicAdd(&p.live[r.root], slots - 1);
     if (old + slots - 1 > p.budget || !coverLive(p, r.root, old + slots - 1)) {
       killRoot(p, r.root);
@@ -1371,15 +1377,16 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
           beam = true;
         }
       }
-      if (groupRootKilled(p, beam, g.r.root)) {
+      const int state = leadState(p, beam, g.r.root);
+      if (beam && g.r.root != qRoot) {
+        loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);
+        qRoot = g.r.root;
+      }
+      if (groupKilled(state)) {
         if (lead) liveSub(p, g.r.root, 1);
         beam = false;
       }
       if (beam) {
-        if (g.r.root != qRoot) {
-          loadRoot<App>(&p.roots[g.r.root], g.q, lightArea);
-          qRoot = g.r.root;
-        }
         g.cx[0] = X.x, g.cx[1] = X.y, g.cx[2] = X.z, g.cx[3] = X.w;
         g.cy[0] = Y.x, g.cy[1] = Y.y, g.cy[2] = Y.z, g.cy[3] = Y.w;
         g.begin(p.s, st);
@@ -1394,12 +1401,7 @@ __global__ void __launch_bounds__(kThreads, kTailCtas) tailGroupKernel(const __g
     } else if (nC >= nS) {
       g.climb(p.s, g.phase == kGClimb, st);
     } else {
-      bool act = g.phase == kGClip;
-      if (groupRootKilled(p, act, g.r.root)) {
-        if (lead) liveSub(p, g.r.root, 1);
-        g.phase = kGIdle;
-        act = false;
-      }
+      const bool act = g.phase == kGClip;
       __syncwarp();
       LanePoly v;
       v.x = g.qx;
@@ -1482,8 +1484,8 @@ __device__ __forceinline__ bool clipQueueFits(const RoundParams& p, int nClip, i
 // vertex each: classifying, splitting and cleaning it are a few ballots and
 // shuffles, where one lane per clip unrolled every polygon step six times
 // behind selects (128 registers with spills, 8 of 32 lanes active, instruction
-// fetch its top stall).  71 registers for soft shadows, 72 for primary beams, 80
-// with 276 bytes of spill stores for point shadows (their occluded pieces are
+// fetch its top stall).  74 registers for soft shadows, 76 for primary beams, 80
+// with 292 bytes of spill stores for point shadows (their occluded pieces are
 // output in the clip); 25.9 KB of shared memory a CTA.  Frames,
 // one lane -> eight lanes per clip (B200): plant 512^2 21.8 -> 18.7 ms, plant
 // 333x217 at light scale 4 49.3 -> 42.1, displaced sphere 512^2 at scale 2
@@ -1504,14 +1506,10 @@ __global__ void __launch_bounds__(kThreads, kClipCtas) clipKernel(const __grid_c
     base = __shfl_sync(kFull, base, 0);
     if (base >= nClip) break;
     const int i = base + (lane >> 3);
-    bool act = i < nClip;
+    const bool act = i < nClip;
     GroupRec r;
     float4 X, Y;
     loadRec(p.cq + min(i, nClip - 1), r, X, Y);
-    if (groupRootKilled(p, act, r.root)) {
-      if (W::sub() == 0) liveSub(p, r.root, 1);
-      act = false;
-    }
     Query q;
     float lightArea;
     loadRoot<App>(&p.roots[r.root], q, lightArea);

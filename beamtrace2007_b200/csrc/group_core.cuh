@@ -50,19 +50,17 @@ struct HitPlane {
   int tri;
 };
 
-// What laneCoefs found: coefficients that makeLine normalises; a constant line
-// (a tie of coplanar surfaces), whose corners vote on its c like any other's;
-// no line at all (lane 3 of a primary record without a hit), which every corner
-// is inside of whatever eps is: eps grows with the root's extent and passes a
-// constant line's 1 in views close to 180 degrees.
-enum LaneLine { kLineNone = 0, kLineConst = 1, kLineCoefs = 2 };
-
 // Edge lines and the depth line of triangle t, one per lane, before they are
-// normalised (BeamCtx::triSetup and closerLine, as testOne evaluates them).
-// `flags`: kTriPlain | kTriFront, the same in all lanes of the group.
+// normalised (BeamCtx::triSetup and closerLine, as testOne evaluates them):
+// true with the coefficients in L, or false with a constant line in L (lane 3).
+// That is a tie of coplanar surfaces, whose corners vote on its 1 or -1 like on
+// any other distance; or no depth line at all -- primary, no hit yet --, which
+// every corner is inside of: infinitely far, whatever eps is (eps grows with the
+// root's extent and passes 1 in views close to 180 degrees).  `flags`: kTriPlain
+// | kTriFront, the same in all lanes of the group.
 template <bool Nearest>
-__device__ __forceinline__ LaneLine laneCoefs(const Query& q, const TriRec& t, const HitPlane& h, Line& L,
-                                              int& flags, V3& r0, V3& r1, V3& r2) {
+__device__ __forceinline__ bool laneCoefs(const Query& q, const TriRec& t, const HitPlane& h, Line& L, int& flags,
+                                          V3& r0, V3& r1, V3& r2) {
   const int e = threadIdx.x & 3;
   r0 = sub(t.v0, q.P.O);
   r1 = sub(t.v1, q.P.O);
@@ -85,8 +83,8 @@ __device__ __forceinline__ LaneLine laneCoefs(const Query& q, const TriRec& t, c
   if (e == 3) {
     constexpr bool far = !Nearest;
     if (!far && h.tri < 0) {
-      L = Line{0.f, 0.f, 1.f};
-      return kLineNone;
+      L = Line{0.f, 0.f, kInf};
+      return false;
     }
     TriInfo ti;
     ti.tri = t.tri;
@@ -97,13 +95,13 @@ __device__ __forceinline__ LaneLine laneCoefs(const Query& q, const TriRec& t, c
     ti.C = dot(t.n, r0);
     const float AF[3] = {far ? 0.f : h.A[0], far ? 0.f : h.A[1], far ? q.farCq : h.A[2]};
     const float CF = far ? q.farCq : h.C;
-    return closerCoefs(ti, AF, CF, far ? q.P.n : h.n, far ? -1 : h.tri, L) ? kLineCoefs : kLineConst;
+    return closerCoefs(ti, AF, CF, far ? q.P.n : h.n, far ? -1 : h.tri, L);
   }
   const float sg = (flags & kTriFront) ? 1.f : -1.f;
   L.a *= sg;
   L.b *= sg;
   L.c *= sg;
-  return kLineCoefs;
+  return true;
 }
 
 // ------------------------------------------------------ the walk of a record
@@ -343,15 +341,14 @@ struct GroupWalk {
     Line L;
     int flags;
     V3 r0, r1, r2;
-    const LaneLine line = laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2);
-    bool anyIn = line == kLineNone || L.c > q.eps, anyOut = L.c < -q.eps;  // (a constant line's vote)
-    const bool known = line != kLineCoefs || voteUnscaled(cx, cy, L.a, L.b, L.c, max4abs(cx), max4abs(cy), q.eps, q.ext,
-                                                          anyIn, anyOut);
+    const bool line = laneCoefs<Nearest>(q, t, h, L, flags, r0, r1, r2);
+    bool anyIn = L.c > q.eps, anyOut = L.c < -q.eps;  // (a constant line's vote)
+    const bool known =
+        !line || voteUnscaled(cx, cy, L.a, L.b, L.c, max4abs(cx), max4abs(cy), q.eps, q.ext, anyIn, anyOut);
     if (__any_sync(0xffffffffu, act && !known)) {
       // a corner too close to its band's edge: the line itself
-      const Line N = line == kLineCoefs ? makeLine(L.a, L.b, L.c, q.ext) : L;
-      anyIn = line == kLineNone;
-      anyOut = false;
+      const Line N = line ? makeLine(L.a, L.b, L.c, q.ext) : L;
+      anyIn = anyOut = false;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float dv = cx[k] * N.a + cy[k] * N.b + N.c;
